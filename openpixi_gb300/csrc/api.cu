@@ -81,7 +81,7 @@ static void release(Ctx &c) {
     super_free(c);
     cgc_vt_free(c);
     void *dev[] = {c.U, c.Unext, c.E, c.J, c.rho, c.active, c.eval, c.staging, c.red_part, c.red_out, c.red_count, c.status,
-                   c.imp_Ua, c.imp_Ub, c.imp_E, c.E_alt, c.W_in, c.W_out, c.meas_part, c.meas_rows, c.bn_site};
+                   c.imp_Ua, c.imp_Ub, c.imp_E, c.E_alt, c.W_in, c.W_out, c.meas_part, c.meas_rows, c.bn_site, c.fx_links};
     for (void *p : dev) if (p) cudaFree(p);
     if (c.red_host) cudaFreeHost(c.red_host);
     if (c.meas_host) cudaFreeHost(c.meas_host);
@@ -131,6 +131,8 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     c.int_offsets = std::getenv("OPX_LONG_OFFSETS") == nullptr && link_elems(V, c.ng) < (1L << 31) - 64 &&
                     3L * c.na * V < (1L << 31);
     c.rsize = c.prec == OPX_F64 ? 8 : 4;
+    c.fixed_kernel = c.prec == OPX_F64 && std::getenv("OPX_FP64_ONLY") == nullptr && c.L.inva2[0] == c.L.inva2[1] &&
+                     c.L.inva2[1] == c.L.inva2[2];
     bool ok = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) == cudaSuccess;
     auto al = [&](void **p, size_t bytes) { if (ok && cudaMalloc(p, bytes) != cudaSuccess) { ok = false; *p = nullptr; } };
     const size_t nU = (size_t)link_elems(V, c.ng), nE = (size_t)V * 3 * c.na;
@@ -150,6 +152,12 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     if (ok && cudaMallocHost((void **)&c.red_host, sizeof(double) * 16) != cudaSuccess) ok = false;
     if (ok && cudaMallocHost((void **)&c.status_host, sizeof(unsigned)) != cudaSuccess) ok = false;
     if (ok && (cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess)) ok = false;
+    // without room for the fixed-point links the handle works all the same, in FP64 products
+    if (ok && c.fixed_kernel && cudaMalloc(&c.fx_links, nU * 8) != cudaSuccess) {
+        cudaGetLastError();
+        c.fx_links = nullptr;
+        c.fixed_kernel = false;
+    }
     if (!ok) {
         release(c);
         delete h;

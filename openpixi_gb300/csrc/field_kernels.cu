@@ -18,6 +18,7 @@
 
 #include "internal.h"
 #include "leapfrog.cuh"
+#include "leapfrog_fx.cuh"
 #include "su3_log.cuh"
 #include "su3_pair.cuh"
 #include "su3_stream.cuh"
@@ -452,11 +453,32 @@ static void launch_update_grid_i(Ctx &c, bool reunit, dim3 grid, int B, const R 
     }
 }
 
+// The FP64 update with its group products in fixed point: the links converted
+// once (SU(2) 128^3: a tenth of the step), then the update.
+template <int NC, typename I>
+static void update_grid_fx(Ctx &c) {
+    const int B = 128;
+    const dim3 grid(grid_for(c.L.V, B));
+    const double *U = (const double *)c.U, *J = (const double *)c.J;
+    double *E = (double *)c.E, *Un = (double *)c.Unext;
+    const int2 *F = (const int2 *)c.fx_links;
+    fx::k_fixed_links<NC><<<dim3(grid.x, 3), B, 0, c.stream>>>(U, (int2 *)c.fx_links, c.L);
+    c.launches += 2;
+    if (c.j_nonzero) fx::k_update_links_fx<NC, true, I><<<3 * grid.x, B, 0, c.stream>>>(F, U, E, J, Un, c.active, c.L);
+    else fx::k_update_links_fx<NC, false, I><<<3 * grid.x, B, 0, c.stream>>>(F, U, E, J, Un, c.active, c.L);
+}
 template <int NC, typename R>
 static void update_grid_t(Ctx &c, bool reunit) {
     if (NC == 3 && sizeof(R) == 4 && c.pair_kernel) {
         update_grid_su3f_pair(c, reunit);
         return;
+    }
+    if constexpr (sizeof(R) == 8) {
+        if (c.fixed_kernel && !reunit) {
+            if (c.int_offsets) update_grid_fx<NC, int>(c);
+            else update_grid_fx<NC, long>(c);
+            return;
+        }
     }
     const int B = 128;
     dim3 grid(grid_for(c.L.V, B));

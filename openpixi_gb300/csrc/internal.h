@@ -70,6 +70,12 @@ struct Ctx {
     // device)
     bool stream_kernel = false;
     int st_grid = 0;
+    // FP64: the group products of the update in fixed point (fixed.cuh) where
+    // the lattice spacings are equal; OPX_FP64_ONLY=1 keeps every product in FP64,
+    // so that tests can compare the two.  fx_links: the links in fixed point, a
+    // workspace that each update fills
+    bool fixed_kernel = true;
+    void *fx_links = nullptr;
     double *staging = nullptr;
     size_t staging_len = 0;  // doubles
     double *red_part = nullptr;
