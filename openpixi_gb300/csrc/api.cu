@@ -25,16 +25,23 @@ static std::string g_create_error;
 
 Ctx &opx::ctx_of(opx_ctx *h) {
     h->c.api_calls++;
+    h->c.links_changed();
     return h->c;
 }
 
 // API_CHECK for entry points that may change the fields or the masks (counted,
-// so that the B^2 reuse of opx_reduce sees them); API_CHECK_RO for the ones
-// that only read.
-#define API_CHECK(ctx)                                   \
+// so that the B^2 reuse of opx_reduce sees them), API_CHECK_STEP for those of
+// them whose kernels and swaps keep track of the fixed-point links themselves;
+// API_CHECK_RO for the ones that only read.
+#define API_CHECK_STEP(ctx)                              \
     do {                                                 \
         if (!(ctx)) return OPX_ERR_INVALID;              \
         (ctx)->c.api_calls++;                            \
+    } while (0)
+#define API_CHECK(ctx)                                   \
+    do {                                                 \
+        API_CHECK_STEP(ctx);                             \
+        (ctx)->c.links_changed();                        \
     } while (0)
 #define API_CHECK_RO(ctx)                                \
     do {                                                 \
@@ -81,7 +88,7 @@ static void release(Ctx &c) {
     super_free(c);
     cgc_vt_free(c);
     void *dev[] = {c.U, c.Unext, c.E, c.J, c.rho, c.active, c.eval, c.staging, c.red_part, c.red_out, c.red_count, c.status,
-                   c.imp_Ua, c.imp_Ub, c.imp_E, c.E_alt, c.W_in, c.W_out, c.meas_part, c.meas_rows, c.bn_site, c.fx_links};
+                   c.imp_Ua, c.imp_Ub, c.imp_E, c.E_alt, c.W_in, c.W_out, c.meas_part, c.meas_rows, c.bn_site, c.fx_U, c.fx_Unext};
     for (void *p : dev) if (p) cudaFree(p);
     if (c.red_host) cudaFreeHost(c.red_host);
     if (c.meas_host) cudaFreeHost(c.meas_host);
@@ -145,7 +152,7 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     c.red_blocks = reduction_blocks(V);
     // 16 doubles per block: the bulk partials, or 2 (slice, split) partials of the projected energy
     al((void **)&c.red_part,
-       sizeof(double) * 2 * BULK_COLUMNS * std::max(c.red_blocks, 2 * c.L.n[0] + 2 * c.L.n[1] + 2 * c.L.n[2]));
+       sizeof(double) * 2 * BULK_COLUMNS * std::max(bulk_blocks_max(V), 2 * c.L.n[0] + 2 * c.L.n[1] + 2 * c.L.n[2]));
     al((void **)&c.red_out, sizeof(double) * 16);
     al((void **)&c.red_count, sizeof(unsigned));
     al((void **)&c.status, sizeof(unsigned));
@@ -153,9 +160,10 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     if (ok && cudaMallocHost((void **)&c.status_host, sizeof(unsigned)) != cudaSuccess) ok = false;
     if (ok && (cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess)) ok = false;
     // without room for the fixed-point links the handle works all the same, in FP64 products
-    if (ok && c.fixed_kernel && cudaMalloc(&c.fx_links, nU * 8) != cudaSuccess) {
+    if (ok && c.fixed_kernel && (cudaMalloc(&c.fx_U, nU * 8) != cudaSuccess || cudaMalloc(&c.fx_Unext, nU * 8) != cudaSuccess)) {
         cudaGetLastError();
-        c.fx_links = nullptr;
+        if (c.fx_U) cudaFree(c.fx_U);
+        c.fx_U = c.fx_Unext = nullptr;
         c.fixed_kernel = false;
     }
     if (!ok) {
@@ -334,7 +342,7 @@ static void phase_end(Ctx &c, int phase) {
 }
 
 int opx_step_links(opx_ctx *ctx) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     phase_begin(c);
     launch_update_links(c);
@@ -343,7 +351,7 @@ int opx_step_links(opx_ctx *ctx) {
 }
 
 int opx_update_grid(opx_ctx *ctx) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     phase_begin(c);
     if (c.imp_solver) {
@@ -357,8 +365,8 @@ int opx_update_grid(opx_ctx *ctx) {
 }
 
 int opx_store_fields(opx_ctx *ctx) {
-    API_CHECK(ctx);
-    std::swap(ctx->c.U, ctx->c.Unext);
+    API_CHECK_STEP(ctx);
+    ctx->c.swap_links();
     return OPX_OK;
 }
 
@@ -379,7 +387,7 @@ static int cpic_ok(Ctx &c, const char *where) {
 }
 
 int opx_cpic_phases(opx_ctx *ctx, int reassign) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     int rc = cpic_ok(c, "opx_cpic_phases");
     if (rc) return rc;
@@ -391,7 +399,7 @@ int opx_cpic_phases(opx_ctx *ctx, int reassign) {
 }
 
 int opx_initialize(opx_ctx *ctx) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     int rc = opx_step_links(ctx);
     if (rc) return rc;
@@ -405,7 +413,7 @@ int opx_initialize(opx_ctx *ctx) {
 
 static int one_step(Ctx &c) {
     c.steps++;
-    std::swap(c.U, c.Unext);  // storeFields
+    c.swap_links();
     const bool reunit = c.prec == OPX_F32 && c.cfg.reunit_every > 0 && (c.steps % c.cfg.reunit_every) == 0;
     phase_begin(c);
     if (c.imp_solver) {
@@ -428,7 +436,7 @@ static int one_step(Ctx &c) {
 }
 
 int opx_step(opx_ctx *ctx, int nsteps) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     if (nsteps < 0) { c.err = "opx_step: nsteps < 0"; return OPX_ERR_INVALID; }
     c.step1_call = nsteps == 1 ? c.api_calls : -1;
@@ -560,7 +568,7 @@ static int ensure_measure_buffers(Ctx &c, int nsteps) {
 }
 
 int opx_step_measured(opx_ctx *ctx, int nsteps, opx_observables *out) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     if (nsteps < 0 || (nsteps > 0 && !out)) { c.err = "opx_step_measured: nsteps < 0 or null output"; return OPX_ERR_INVALID; }
     if (nsteps == 0) return OPX_OK;
@@ -581,7 +589,7 @@ int opx_step_measured(opx_ctx *ctx, int nsteps, opx_observables *out) {
         phase_begin(c);
         for (int k = 0; k < nk; k++) {
             c.steps++;
-            std::swap(c.U, c.Unext);  // storeFields
+            c.swap_links();
             const bool reunit = c.cfg.reunit_every > 0 && (c.steps % c.cfg.reunit_every) == 0;
             launch_update_measure(c, reunit, c.E_alt, c.W_in, c.W_out, c.meas_part + per_step * k);
             std::swap(c.E, c.E_alt);
@@ -889,7 +897,7 @@ int opx_phase_times(opx_ctx *ctx, double *ms, long *counts, int nphases) {
 }
 
 int opx_time_steps(opx_ctx *ctx, int nsteps, double *ms) {
-    API_CHECK(ctx);
+    API_CHECK_STEP(ctx);
     Ctx &c = ctx->c;
     if (nsteps < 0 || !ms) { c.err = "opx_time_steps: invalid arguments"; return OPX_ERR_INVALID; }
     const bool prof = c.profiling;

@@ -319,6 +319,7 @@ static int implicit_update_t(Ctx &c) {
             return OPX_ERR_NOMEM;
         }
     }
+    c.fx_Unext_ok = false;
     R *Ui = (R *)c.imp_Ua, *Uin = (R *)c.imp_Ub, *Ei = (R *)c.imp_E;
     // Grid(grid): the implicit grid starts as a copy
     cudaMemcpyAsync(Ui, c.U, nU, cudaMemcpyDeviceToDevice, c.stream);
@@ -453,19 +454,34 @@ static void launch_update_grid_i(Ctx &c, bool reunit, dim3 grid, int B, const R 
     }
 }
 
-// The FP64 update with its group products in fixed point: the links converted
-// once (SU(2) 128^3: a tenth of the step), then the update.
+void ensure_fixed_links(Ctx &c, bool u, bool unext) {
+    const dim3 grid(grid_for(c.L.V, 128), 3);
+    auto fill = [&](const void *links, void *out, bool &ok) {
+        if (ok) return;
+        if (c.nc == 2) fx::k_fixed_links<2><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
+        else fx::k_fixed_links<3><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
+        c.launches++;
+        ok = true;
+    };
+    if (u) fill(c.U, c.fx_U, c.fx_U_ok);
+    if (unext) fill(c.Unext, c.fx_Unext, c.fx_Unext_ok);
+}
+
+// The FP64 update with its group products in fixed point; it leaves Unext in
+// both forms (with a mask, the cells that it skips keep older links: converted
+// again when they are wanted)
 template <int NC, typename I>
 static void update_grid_fx(Ctx &c) {
-    const int B = 128;
-    const dim3 grid(grid_for(c.L.V, B));
+    const int B = 128, nb = 3 * grid_for(c.L.V, B);
     const double *U = (const double *)c.U, *J = (const double *)c.J;
     double *E = (double *)c.E, *Un = (double *)c.Unext;
-    const int2 *F = (const int2 *)c.fx_links;
-    fx::k_fixed_links<NC><<<dim3(grid.x, 3), B, 0, c.stream>>>(U, (int2 *)c.fx_links, c.L);
-    c.launches += 2;
-    if (c.j_nonzero) fx::k_update_links_fx<NC, true, I><<<3 * grid.x, B, 0, c.stream>>>(F, U, E, J, Un, c.active, c.L);
-    else fx::k_update_links_fx<NC, false, I><<<3 * grid.x, B, 0, c.stream>>>(F, U, E, J, Un, c.active, c.L);
+    ensure_fixed_links(c, true, false);
+    const int2 *F = (const int2 *)c.fx_U;
+    int2 *Fn = (int2 *)c.fx_Unext;
+    if (c.j_nonzero) fx::k_update_links_fx<NC, true, I><<<nb, B, 0, c.stream>>>(F, U, E, J, Un, Fn, c.active, c.L);
+    else fx::k_update_links_fx<NC, false, I><<<nb, B, 0, c.stream>>>(F, U, E, J, Un, Fn, c.active, c.L);
+    c.fx_Unext_ok = c.active == nullptr;
+    c.launches++;
 }
 template <int NC, typename R>
 static void update_grid_t(Ctx &c, bool reunit) {
@@ -480,6 +496,7 @@ static void update_grid_t(Ctx &c, bool reunit) {
             return;
         }
     }
+    c.fx_Unext_ok = false;
     const int B = 128;
     dim3 grid(grid_for(c.L.V, B));
     const R *U = (const R *)c.U;
@@ -500,6 +517,7 @@ void launch_update_grid(Ctx &c, bool reunit) {
 
 template <int NC, typename R>
 static void update_links_t(Ctx &c) {
+    c.fx_Unext_ok = false;
     const int B = 128;
     k_update_links<NC, R><<<grid_for(c.L.V, B), B, 0, c.stream>>>((const R *)c.U, (const R *)c.E,
                                                                    (R *)c.Unext, c.active, c.L);

@@ -50,10 +50,18 @@ constexpr i64 HALF30 = 1LL << 29, ONE30 = 1LL << 30;
 // of one that value() ends (rounded)
 OPX_HD OPX_INLINE Acc acc0() { return Acc{HALF30, HALF30}; }
 OPX_HD OPX_INLINE Acc acc0v() { return Acc{0, HALF30}; }
+// (asm: the compiler would turn a product with a negated factor into a product
+// and a 64-bit subtraction, three instructions for one)
 OPX_HD OPX_INLINE void mac(Acc &s, Fx x, Fx y) {
+#ifdef __CUDA_ARCH__
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s.a) : "r"(x.h), "r"(y.h));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s.b) : "r"(x.h), "r"(y.l));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s.b) : "r"(x.l), "r"(y.h));
+#else
     s.a += (i64)x.h * y.h;
     s.b += (i64)x.h * y.l;
     s.b += (i64)x.l * y.h;
+#endif
 }
 OPX_HD OPX_INLINE Fx neg(Fx x) { return Fx{-x.h, -x.l}; }
 // F + 2^30 (F in units of 2^-61) to (h, l)
@@ -259,34 +267,63 @@ template <bool CA, bool CB> OPX_HD OPX_INLINE void mmul(M &c, const M &a, const 
             c.i[3 * r + q] = pack(t);
         }
 }
-// S += A B in units of 2^-60: S[k] real, S[9 + k] imaginary
-template <bool CA, bool CB> OPX_HD OPX_INLINE void macc(i64 *S, const M &a, const M &b) {
+// A row of a matrix.  The SU(3) kernels form products row by row, v -> v B, in a
+// loop over the three rows, with B's entries read from the link arrays as they are
+// used: a third of the code of whole matrix products (which overran the
+// instruction cache and 168 registers).
+struct Row {
+    Fx r[3], i[3];
+};
+// component q of v B or (CB) v B^dagger; B(c) gives B's entry c = 3 row + column as (real, imaginary)
+template <bool CB, class B> OPX_HD OPX_INLINE void rterm(Acc &re, Acc &im, const Row &v, const B &b, int q) {
 #pragma unroll
-    for (int r = 0; r < 3; r++)
+    for (int k = 0; k < 3; k++) {
+        Fx br, bi;
+        b(CB ? 3 * q + k : 3 * k + q, br, bi);
+        mac(re, v.r[k], br);
+        mac(re, CB ? v.i[k] : neg(v.i[k]), bi);
+        mac(im, CB ? neg(v.r[k]) : v.r[k], bi);
+        mac(im, v.i[k], br);
+    }
+}
+template <bool CB, class B> OPX_HD OPX_INLINE Row rmul(const Row &v, const B &b) {
+    Row o;
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            Acc s{S[3 * r + q], ONE30}, t{S[9 + 3 * r + q], ONE30};
-            mre<CA, CB>(s, a, b, r, q);
-            mim<CA, CB>(t, a, b, r, q);
-            S[3 * r + q] = s.a + (s.b >> 31);
-            S[9 + 3 * r + q] = t.a + (t.b >> 31);
-        }
+    for (int q = 0; q < 3; q++) {
+        Acc re = acc0(), im = acc0();
+        rterm<CB>(re, im, v, b, q);
+        o.r[q] = pack(re);
+        o.i[q] = pack(im);
+    }
+    return o;
 }
-// proj_a(A B) = Im tr(lambda_a A B) for a = 0..6, and the eighth component times
-// sqrt(3) / 2, in the units of the product (value()); only the entries proj reads
-template <bool CA, bool CB> OPX_HD OPX_INLINE void mproj(i64 *x, const M &a, const M &b) {
-    auto re = [&](int r, int q) { Acc s = acc0v(); mre<CA, CB>(s, a, b, r, q); return value(s); };
-    auto im = [&](int r, int q) { Acc s = acc0v(); mim<CA, CB>(s, a, b, r, q); return value(s); };
-    x[0] = im(0, 1) + im(1, 0);
-    x[1] = re(0, 1) - re(1, 0);
-    x[3] = im(0, 2) + im(2, 0);
-    x[4] = re(0, 2) - re(2, 0);
-    x[5] = im(1, 2) + im(2, 1);
-    x[6] = re(1, 2) - re(2, 1);
-    const i64 d0 = im(0, 0), d1 = im(1, 1), d2 = im(2, 2);
-    x[2] = d0 - d1;
-    x[7] = ((d0 + d1) >> 1) - d2;
+// S += v B in units of 2^-60: S[q] real, S[3 + q] imaginary
+template <bool CB, class B> OPX_HD OPX_INLINE void racc(i64 *S, const Row &v, const B &b) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        Acc re{S[q], ONE30}, im{S[3 + q], ONE30};
+        rterm<CB>(re, im, v, b, q);
+        S[q] = re.a + (re.b >> 31);
+        S[3 + q] = im.a + (im.b >> 31);
+    }
 }
+// Adds row r of a matrix (entries re, im in any one unit) to x_a = Im tr(lambda_a
+// M), a < 7; x_7 collects the imaginary diagonal as its own three sums do: d0 + d1 in
+// x_7, d2 in x_8
+OPX_HD OPX_INLINE void proj_row(i64 *x, int r, const i64 *re, const i64 *im) {
+    if (r == 0) {
+        x[0] += im[1]; x[1] += re[1]; x[3] += im[2]; x[4] += re[2];
+        x[2] += im[0]; x[7] += im[0];
+    } else if (r == 1) {
+        x[0] += im[0]; x[1] -= re[0]; x[5] += im[2]; x[6] += re[2];
+        x[2] -= im[1]; x[7] += im[1];
+    } else {
+        x[3] += im[0]; x[4] -= re[0]; x[5] += im[1]; x[6] -= re[1];
+        x[8] += im[2];
+    }
+}
+// the eighth component times sqrt(3) / 2 (the halved sum stays in range)
+OPX_HD OPX_INLINE i64 proj_eighth(const i64 *x) { return (x[7] >> 1) - x[8]; }
 
 // exp(i H), H = v_a lambda_a / 2, from t_a = (v_a / 2) 2^61 (a < 7) and t_7 =
 // (v_7 / (2 sqrt 3)) 2^61; false where an entry reaches 1/2 (or is not finite) or
@@ -482,9 +519,39 @@ template <typename I> struct FxLinks<2, I> {
         return Q{{{x.y, x.x}, {x.w, x.z}, {y.y, y.x}, {y.w, y.z}}};
     }
 };
+// the entries of one link in memory
+struct FxEntries {
+    const int2 *b;
+    __device__ __forceinline__ Fx at(int c) const {
+        const int2 x = __ldg(b + 32 * c);
+        return Fx{x.y, x.x};
+    }
+    __device__ __forceinline__ void operator()(int c, Fx &re, Fx &im) const {
+        re = at(c);
+        im = at(9 + c);
+    }
+    // row r, and row r of the adjoint
+    __device__ __forceinline__ Row row(int r) const {
+        Row v;
+#pragma unroll
+        for (int k = 0; k < 3; k++) (*this)(3 * r + k, v.r[k], v.i[k]);
+        return v;
+    }
+    __device__ __forceinline__ Row adj_row(int r) const {
+        Row v;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            (*this)(3 * k + r, v.r[k], v.i[k]);
+            v.i[k] = neg(v.i[k]);
+        }
+        return v;
+    }
+    __device__ __forceinline__ int mark() const { return __ldg(b).y; }  // h of the first entry: LINK_BAD or not
+};
 template <typename I> struct FxLinks<3, I> {
     const int2 *p;
     I V;
+    __device__ __forceinline__ FxEntries at(int d, I s) const { return FxEntries{p + link_offset_t<I>(V, 18, d, 0, s)}; }
     __device__ __forceinline__ M load(int d, I s) const {
         const int2 *b = p + link_offset_t<I>(V, 18, d, 0, s);
         M m;
@@ -498,20 +565,19 @@ template <typename I> struct FxLinks<3, I> {
     }
 };
 
-// One link per thread: the FP64 links in fixed point (k = link index d V + s)
-template <int NC>
-__global__ void __launch_bounds__(128) k_fixed_links(const double *__restrict__ U, int2 *__restrict__ out, Lat L) {
+// Link (d, s) of U in fixed point into out
+template <int NC, typename I>
+__device__ __forceinline__ void fixed_link(const double *U, int2 *out, I V, int d, I s) {
     constexpr int NG = LinkOf<NC>::NG;
-    const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= L.V) return;
-    const int d = blockIdx.y;
     double u[NG];
-    const long o = link_offset(L.V, NG, d, 0, s);
+    const I o = link_offset_t<I>(V, NG, d, 0, s);
     if constexpr (NC == 2) {
-        ld4<double>(U + o, u);
+        const double2 *b = reinterpret_cast<const double2 *>(U + o);
+        const double2 x = b[0], y = b[1];
+        u[0] = x.x; u[1] = x.y; u[2] = y.x; u[3] = y.y;
     } else {
 #pragma unroll
-        for (int c = 0; c < NG; c++) u[c] = __ldg(U + o + 32 * c);
+        for (int c = 0; c < NG; c++) u[c] = U[o + 32 * c];
     }
     auto m = link_of<NC>(u);
     if constexpr (NC == 2) {
@@ -525,6 +591,13 @@ __global__ void __launch_bounds__(128) k_fixed_links(const double *__restrict__ 
             out[o + 32 * c] = make_int2(x.l, x.h);
         }
     }
+}
+
+// One link per thread (blockIdx.y its direction)
+template <int NC>
+__global__ void __launch_bounds__(128) k_fixed_links(const double *__restrict__ U, int2 *__restrict__ out, Lat L) {
+    const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < L.V) fixed_link<NC, long>(U, out, L.V, (int)blockIdx.y, s);
 }
 #endif
 

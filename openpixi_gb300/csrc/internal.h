@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/opixi.h"
@@ -70,12 +71,21 @@ struct Ctx {
     // device)
     bool stream_kernel = false;
     int st_grid = 0;
-    // FP64: the group products of the update in fixed point (fixed.cuh) where
-    // the lattice spacings are equal; OPX_FP64_ONLY=1 keeps every product in FP64,
-    // so that tests can compare the two.  fx_links: the links in fixed point, a
-    // workspace that each update fills
+    // FP64: the group products of the update and the reductions in fixed point
+    // (fixed.cuh) where the lattice spacings are equal; OPX_FP64_ONLY=1 keeps every
+    // product in FP64, so that tests can compare the two.  fx_U, fx_Unext: U and
+    // Unext in fixed point beside the doubles (swapped with them); fx_*_ok: whether
+    // they hold the present links (cleared by every entry point that may write
+    // links otherwise than the fixed-point update does)
     bool fixed_kernel = true;
-    void *fx_links = nullptr;
+    void *fx_U = nullptr, *fx_Unext = nullptr;
+    bool fx_U_ok = false, fx_Unext_ok = false;
+    void links_changed() { fx_U_ok = fx_Unext_ok = false; }
+    void swap_links() {  // storeFields
+        std::swap(U, Unext);
+        std::swap(fx_U, fx_Unext);
+        std::swap(fx_U_ok, fx_Unext_ok);
+    }
     double *staging = nullptr;
     size_t staging_len = 0;  // doubles
     double *red_part = nullptr;
@@ -146,6 +156,7 @@ void launch_update_grid(Ctx &c, bool reunit);
 int launch_implicit_update(Ctx &c);  // ImplicitTYMSolver.step in place of launch_update_grid
 void launch_update_links(Ctx &c);
 void launch_reunit(Ctx &c, void *links);
+void ensure_fixed_links(Ctx &c, bool u, bool unext);  // fx_U / fx_Unext of the present links
 // the measured step (SU(3) FP32 paired form, FastTYMSolver, no current, no
 // masks, no particles): row[0..6] = E^2 of the new E [3] (x (g a_i)^-2),
 // B^2 of the step's input links [3] (x (g a_i)^-2 / 2), G^2 of the state
@@ -161,6 +172,7 @@ void launch_measure_combine(Ctx &c, const double *part, int nsteps, double *rows
 constexpr int BULK_COLUMNS = 11;
 void launch_bulk(Ctx &c, int skip_u);
 int reduction_blocks(long V);
+int bulk_blocks_max(long V);
 void launch_energy_density(Ctx &c, double *dev_out);
 // six rows of dims[dir]: T_el, T_mag(U), L_el, L_mag(U), T_mag(Unext), L_mag(Unext)
 // (the U rows zero with skip_u); with bn_site the per-site B^2 of Unext come

@@ -31,6 +31,8 @@ struct Lat {
     // precisions, so that FP32 kernels do no FP64 arithmetic or conversions
     double inva2[3], jfac[3];
     float inva2f[3], jfacf[3], dtf;
+    // (g a_i)^-2, the unit factor of squared fields
+    double ufac[3];
     // Grid.getB area factor a_d / (a_j a_k) and Gauss-law factor 1 / (a_i g a_i)
     double bfac[3], gfac[3];
     float bfacf[3], gfacf[3];
@@ -63,6 +65,7 @@ __host__ inline Lat make_lat(const int *dims, const double *a, double dt, double
     for (int i = 0; i < 3; i++) {
         L.inva2[i] = 1.0 / (a[i] * a[i]);
         L.jfac[i] = -(g * a[i]) * dt;
+        L.ufac[i] = 1.0 / ((g * a[i]) * (g * a[i]));
         L.inva2f[i] = (float)L.inva2[i];
         L.jfacf[i] = (float)L.jfac[i];
     }

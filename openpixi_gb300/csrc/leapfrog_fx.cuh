@@ -12,12 +12,14 @@
 // closer to the identity than 2^-7 in every entry (fixed.cuh: there the FP64
 // product is the more exact one); the caller then makes the FP64 update.
 //
-// Bound: the integer pipe.  128^3 SU(2) 2.014 -> 0.728 ms a step, SU(3) 96^3
-// 9.79 -> 2.65 ms (the FP64 pipe before); 32^3 0.041 -> 0.021 ms and SU(3) 16^3
-// 0.221 -> 0.039 ms, where a thread's serial chain counts: one link per thread
-// is a third of it, and beats one site per thread with the forward staples of a
-// plane sharing a product (21 instead of 24 products for a site) at every size
-// (SU(2): 16^3 0.0123 against 0.0184 ms, 128^3 0.728 against 0.773).
+// Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.291 ms
+// a step, SU(3) 64^3 2.99 -> 0.492 ms (the FP64 pipe before); 32^3 0.041 -> 0.018 ms
+// and SU(3) 16^3 0.221 -> 0.027 ms, where a thread's serial chain counts: one link
+// per thread is a third of it, and beats one site per thread with the forward
+// staples of a plane sharing a product (21 instead of 24 products for a site) at
+// every size tried (SU(2) 16^3 0.0123 against 0.0184 ms, 128^3 0.728 against 0.773).
+// SU(3) by whole matrix products at 168 registers: 64^3 0.727 against 0.681 ms row
+// by row at 128 (both before the multiply-adds were written in asm, 0.492).
 #pragma once
 #include "fixed.cuh"
 #include "leapfrog.cuh"
@@ -28,7 +30,7 @@ namespace fx {
 // Unext of one link from its new E where qexp / mexp refuses (a large or
 // non-finite dt E): the FP64 exponential and product
 template <int NC, typename I>
-__device__ __noinline__ void link_update_f64(const double *__restrict__ U, double *__restrict__ Un, const Lat &L, I s, int i,
+__device__ __forceinline__ void link_update_f64(const double *__restrict__ U, double *__restrict__ Un, const Lat &L, I s, int i,
                                              const double *e) {
     using G = typename GroupOf<NC, double>::T;
     double v[G::NA];
@@ -83,7 +85,7 @@ __device__ __forceinline__ void finish_link(const Q &Ui, const i64 *S, const dou
 
 // The FP64 update of one link (the staples in the order of update_site)
 template <int NC, bool HAS_J, typename I>
-__device__ __noinline__ void update_link_f64(const double *__restrict__ U, double *__restrict__ E, const double *__restrict__ J,
+__device__ __forceinline__ void update_link_f64(const double *__restrict__ U, double *__restrict__ E, const double *__restrict__ J,
                                              double *__restrict__ Unext, const Lat &L, I s, int i) {
     using G = typename GroupOf<NC, double>::T;
     using MM = typename G::M;
@@ -155,8 +157,8 @@ __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double 
     return true;
 }
 
-// SU(3), one link; the loop over the staple plane rolled (an unrolled body does
-// not fit the instruction cache)
+// SU(3), one link: the staple sum row by row, the loops over the row and the
+// staple plane rolled
 template <bool HAS_J, typename I>
 __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double *__restrict__ U, double *__restrict__ E,
                                             const double *__restrict__ J, double *__restrict__ Unext, const Lat &L, I s, int i) {
@@ -181,32 +183,54 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
     if (worst == LINK_BAD || offdiag(W.load(i, s)) < WEAK_H) return false;
     const AlgPlanes<8, double, I> Ep{E, (I)L.V}, Jp{const_cast<double *>(J), (I)L.V};
     const LinkPlanes<SU3<double>, double, I> Un{Unext, (I)L.V};
-    const double kdt = L.dt * L.inva2[0] * 0x1p-59, kv = L.dt * -0x1p60;
-    i64 S[18];
+    const double kdt = L.dt * L.inva2[0] * 0x1p-58, kv = L.dt * -0x1p60;
+    const FxEntries Ui = W.at(i, s);
+    // U_i S, S's rows one by one: proj in units of 2^-58
+    i64 x9[9];
 #pragma unroll
-    for (int c = 0; c < 18; c++) S[c] = 0;
+    for (int a = 0; a < 9; a++) x9[a] = 0;
 #pragma unroll 1
-    for (int jj = 1; jj < 3; jj++) {
-        const int j = i + jj >= 3 ? i + jj - 3 : i + jj;
-        const I bj = D.b(j);
-        M T;
-        mmul<false, true>(T, W.load(j, pi), W.load(i, s + D.f(j)));
-        macc<false, true>(S, T, W.load(j, s));
-        mmul<false, false>(T, W.load(i, s + bj), W.load(j, pi + bj));
-        macc<true, false>(S, T, W.load(j, s + bj));
+    for (int r = 0; r < 3; r++) {
+        i64 S[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+        for (int jj = 1; jj < 3; jj++) {
+            const int j = i + jj >= 3 ? i + jj - 3 : i + jj;
+            const I bj = D.b(j);
+            // U_j(x+i) U_i(x+j)^dagger U_j(x)^dagger
+            racc<true>(S, rmul<true>(W.at(j, pi).row(r), W.at(i, s + D.f(j))), W.at(j, s));
+            // U_j(x+i-j)^dagger U_i(x-j)^dagger U_j(x-j)
+            racc<false>(S, rmul<true>(W.at(j, pi + bj).adj_row(r), W.at(i, s + bj)), W.at(j, s + bj));
+        }
+        Row F;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            F.r[q] = quarter(S[q]);
+            F.i[q] = quarter(S[3 + q]);
+        }
+        // entry (p, q) of U_i S gains U_i(p, r) S(r, q)
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            Fx ur, ui;
+            Ui(3 * p + r, ur, ui);
+            i64 re[3], im[3];
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                Acc a{0, ONE30}, b{0, ONE30};
+                mac(a, ur, F.r[q]);
+                mac(a, neg(ui), F.i[q]);
+                mac(b, ur, F.i[q]);
+                mac(b, ui, F.r[q]);
+                re[q] = a.a + (a.b >> 31);
+                im[q] = b.a + (b.b >> 31);
+            }
+            proj_row(x9, p, re, im);
+        }
     }
     double e[8], t[8];
-    {
-        M F;
+    Ep.load(i, s, e);
 #pragma unroll
-        for (int c = 0; c < 18; c++) entry(F, c) = quarter(S[c]);
-        i64 p[8];
-        mproj<false, false>(p, W.load(i, s), F);
-        Ep.load(i, s, e);
-#pragma unroll
-        for (int a = 0; a < 7; a++) e[a] = fma((double)p[a], kdt, e[a]);
-        e[7] = fma((double)p[7], kdt * 1.15470053837925152902, e[7]);  // 2 / sqrt 3
-    }
+    for (int a = 0; a < 7; a++) e[a] = fma((double)x9[a], kdt, e[a]);
+    e[7] = fma((double)proj_eighth(x9), kdt * 1.15470053837925152902, e[7]);  // 2 / sqrt 3
     if (HAS_J) {
         double jv[8];
         Jp.load_ro(i, s, jv);
@@ -220,18 +244,20 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
     t[7] = kv * 0.57735026918962576451 * e[7];
     M X;
     if (mexp(t, X)) {
-        const M Ui = W.load(i, s);
         M3<double> V;
 #pragma unroll
-        for (int r = 0; r < 3; r++)
+        for (int r = 0; r < 3; r++) {
+            Row v;
+#pragma unroll
+            for (int k = 0; k < 3; k++) { v.r[k] = X.r[3 * r + k]; v.i[k] = X.i[3 * r + k]; }
 #pragma unroll
             for (int q = 0; q < 3; q++) {
                 Acc a = acc0v(), b = acc0v();
-                mre<false, false>(a, X, Ui, r, q);
-                mim<false, false>(b, X, Ui, r, q);
+                rterm<false>(a, b, v, Ui, q);
                 V.r[3 * r + q] = double_of(value(a));
                 V.i[3 * r + q] = double_of(value(b));
             }
+        }
         Un.store(i, s, V);
     } else {
         link_update_f64<3, I>(U, Unext, L, s, i, e);
@@ -241,12 +267,12 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
 
 // One link per thread, the three links of 128 sites in three consecutive blocks
 template <int NC> struct FxBounds { static constexpr int minb = 5; };
-template <> struct FxBounds<3> { static constexpr int minb = 3; };
+template <> struct FxBounds<3> { static constexpr int minb = 4; };
 template <int NC, bool HAS_J, typename I>
 __global__ void __launch_bounds__(128, FxBounds<NC>::minb)
 k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, double *__restrict__ E,
-                  const double *__restrict__ J, double *__restrict__ Unext, const uint8_t *__restrict__ active,
-                  const __grid_constant__ Lat L) {
+                  const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf,
+                  const uint8_t *__restrict__ active, const __grid_constant__ Lat L) {
     const unsigned chunk = blockIdx.x / 3u;
     const int i = (int)(blockIdx.x - 3u * chunk);
     const I s = (I)chunk * (I)blockDim.x + (I)threadIdx.x;
@@ -254,6 +280,8 @@ k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, dou
     if (active && !active[s]) return;  // Cell.isActive gate (FastTYMSolver.java:51)
     if (!update_link<HAS_J, I>(FxLinks<NC, I>{Uf, (I)L.V}, U, E, J, Unext, L, s, i))
         update_link_f64<NC, HAS_J, I>(U, E, J, Unext, L, s, i);
+    // the new link in fixed point, from the double that was stored
+    fixed_link<NC, I>(Unext, Unf, (I)L.V, i, s);
 }
 
 }  // namespace fx

@@ -3,6 +3,7 @@
 #pragma once
 #include "ksum.cuh"
 #include "lattice.cuh"
+#include "transport_fx.cuh"
 
 namespace opx {
 
@@ -102,7 +103,41 @@ __device__ __forceinline__ void bulk_accumulate(const R *__restrict__ U, const R
             else { p[2] += ev; p[5] += bv; }
         }
         R gs[NA];
-        gauss_site<G, R>(Up, Ep, rho, L, s, nb, gs);
+        if constexpr (sizeof(R) == 8) {
+            // the transports of opx_reduce (k_bulk_partial_fx), bit for bit
+            if (L.inva2[0] == L.inva2[1] && L.inva2[1] == L.inva2[2]) {
+#pragma unroll
+                for (int a = 0; a < NA; a++) gs[a] = 0.0;
+#pragma unroll 1
+                for (int i = 0; i < 3; i++) {
+                    const long sm = pick3(nb.bwd[0], nb.bwd[1], nb.bwd[2], i);
+                    const auto Ub = Up.load(i, sm);
+                    double u[G::NG];
+                    if constexpr (NC == 2) {
+#pragma unroll
+                        for (int c = 0; c < 4; c++) u[c] = Ub.e[c];
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 9; c++) { u[c] = Ub.r[c]; u[9 + c] = Ub.i[c]; }
+                    }
+                    double r[NA];
+                    const auto Uf = fx::link_of<NC>(u);
+                    if constexpr (NC == 2) fx::gauss_term<NC, long>(Uf, fx::transportable(Uf), U, E, L, s, sm, i, r);
+                    else fx::gauss_term<NC, long>(fx::HeldEntries{Uf}, fx::transportable(Uf), U, E, L, s, sm, i, r);
+                    const double f = LatR<double>::gfac(L, i);
+#pragma unroll
+                    for (int a = 0; a < NA; a++) gs[a] = fma(r[a], f, gs[a]);
+                }
+                if (rho) {
+#pragma unroll
+                    for (int a = 0; a < NA; a++) gs[a] -= __ldg(rho + (long)a * L.V + s);
+                }
+            } else {
+                gauss_site<G, R>(Up, Ep, rho, L, s, nb, gs);
+            }
+        } else {
+            gauss_site<G, R>(Up, Ep, rho, L, s, nb, gs);
+        }
         p[6] += sqr<R, NA>(gs);
         if (rho) {
             R r[NA];

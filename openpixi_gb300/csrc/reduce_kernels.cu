@@ -9,6 +9,8 @@
 //       storage) or in FP32 Kahan runs added to an FP64 sum (FP32 storage); a
 //       block adds its threads in a fixed FP64 tree and the block partials are
 //       combined by one block in a fixed order, so results are deterministic.
+//   k_bulk_partial_fx  : the same for FP64 storage with the group products in
+//       fixed point (fixed.cuh), four threads a site
 //   k_energy_density   : EnergyDensity.ComponentComputation (EnergyDensity.java:119-166)
 //   k_projected_energy : ProjectedEnergyDensity.EnergyDensityComputation (:114-179)
 //   k_gauss_field      : Grid.getGaussConstraint (Grid.java:944-968) at every cell
@@ -17,6 +19,7 @@
 #include "internal.h"
 #include "ksum.cuh"
 #include "observables.cuh"
+#include "reduce_fx.cuh"
 #include "su3_pair.cuh"
 
 namespace opx {
@@ -35,9 +38,8 @@ constexpr int RED_THREADS = 128;
 constexpr int NQS = BULK_COLUMNS;
 
 // The last block of a reduction to finish combines the block partials: warp w
-// takes columns w, w + nwarps, ...; its lanes stride over the blocks with
-// compensated sums and a fixed shuffle tree adds the lanes.  So a reduction is
-// one launch.  Each block publishes its partials, fences and draws a ticket;
+// takes columns w, w + nwarps, ... and sums them over the blocks with aligned
+// integer mantissas (warp_sum_pairs).  So a reduction is one launch.  Each block publishes its partials, fences and draws a ticket;
 // the block that draws the last ticket reads every partial (through L2) and
 // resets the counter for the next launch on the stream.  No block waits on
 // another.
@@ -52,14 +54,8 @@ __device__ __forceinline__ void last_block_combine(const double *part, unsigned 
     __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
     for (int q = warp; q < NQ; q += nw) {
-        KSum v{0.0, 0.0};
-        for (int b = lane; b < (int)gridDim.x; b += 32)
-            ksum_merge(v, KSum{__ldcg(part + ((long)b * NQ + q) * 2), __ldcg(part + ((long)b * NQ + q) * 2 + 1)});
-        for (int o = 16; o > 0; o >>= 1) {
-            KSum w{__shfl_down_sync(0xffffffffu, v.s, o), __shfl_down_sync(0xffffffffu, v.c, o)};
-            ksum_merge(v, w);
-        }
-        if (lane == 0) out[q] = v.s + v.c;
+        const double v = warp_sum_pairs(part + 2 * q, (int)gridDim.x, 2L * NQ);
+        if (lane == 0) out[q] = v;
     }
     if (threadIdx.x == 0) *count = 0u;
 }
@@ -139,6 +135,107 @@ __global__ void __launch_bounds__(RED_THREADS, RedBounds<NC, R>::minb)
     last_block_combine<NQS>(part, count, out);
 }
 
+// FP64 with the group products in fixed point.  Three warps share 32 sites, warp d
+// of them taking E_d^2, B_d^2 and the Gauss law's term of direction d; the terms
+// meet in shared memory (double-buffered, one barrier of the three warps a
+// round), where warp d sums and squares the components d, d + 3, ...  A thread's serial
+// chain is then a third of the site's, which is what a small lattice waits for,
+// and the warps are equally busy (a fourth warp for the whole Gauss law held the
+// other three at the end: 0.373 against 0.245 ms at 256 x 64^2).  Per-site
+// values are summed in FP64 in runs of 32 that are folded into TwoSum-compensated
+// sums, the lanes and blocks by warp_sum.
+template <int NC> struct BulkFx { static constexpr int groups = 2, minb = 3; };
+template <> struct BulkFx<3> { static constexpr int groups = 1, minb = 4; };
+
+template <int NC, typename I>
+__global__ void __launch_bounds__(BulkFx<NC>::groups * 96, BulkFx<NC>::minb)
+    k_bulk_partial_fx(const int2 *__restrict__ Uf, const int2 *__restrict__ Unf, const double *__restrict__ U,
+                      const double *__restrict__ Unext, const double *__restrict__ E, const double *__restrict__ rho,
+                      const uint8_t *__restrict__ eval, const __grid_constant__ Lat L, int skip_u,
+                      double *__restrict__ part, unsigned *__restrict__ count, double *__restrict__ out,
+                      double *__restrict__ bn_site) {
+    constexpr int NA = NC == 2 ? 3 : 8, G = BulkFx<NC>::groups;
+    __shared__ double sh[5][3 * G];
+    __shared__ double gt[2][G][3][NA][32];
+    const int lane = threadIdx.x & 31, d = (threadIdx.x >> 5) % 3, group = threadIdx.x / 96;
+    const I ngroups = (I)((L.V + 31) >> 5);
+    const AlgPlanes<NA, double, I> Ep{const_cast<double *>(E), (I)L.V};
+    // E_d^2, B_d(U)^2, B_d(Unext)^2, G^2 and rho^2 of this warp's components
+    KSum acc[5] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    double p[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    int run = 0;
+    for (I g = (I)blockIdx.x * G + group; g < ngroups; g += (I)gridDim.x * G) {
+        const I s = g * 32 + lane;
+        const bool on = s < (I)L.V && (!eval || eval[s]);
+        if (on) {
+            int x[3];
+            site_coords<I>(L, s, x);
+            const Deltas<I> D = deltas<I>(L, x);
+            double e[NA], r[NA];
+            Ep.load_ro(d, s, e);
+            p[0] += sqr<double, NA>(e);
+            const fx::FxLinks<NC, I> W{Uf, (I)L.V};
+            // one body for both times (the code of two does not fit the instruction cache)
+#pragma unroll 1
+            for (int tt = skip_u ? 1 : 0; tt < 2; tt++) {
+                const double b = fx::plane_b2<I>(fx::FxLinks<NC, I>{tt ? Unf : Uf, (I)L.V}, tt ? Unext : U, L, s, x, D, d);
+                if (tt == 0) {
+                    p[1] += b;
+                } else {
+                    if (bn_site) bn_site[(long)d * L.V + s] = b;
+                    p[2] += b;
+                }
+            }
+            const I sm = s + D.b(d);
+            const auto Ub = W.load(d, sm);
+            if constexpr (NC == 2) fx::gauss_term<NC, I>(Ub, fx::transportable(Ub), U, E, L, s, sm, d, r);
+            else fx::gauss_term<NC, I>(W.at(d, sm), fx::transportable(Ub), U, E, L, s, sm, d, r);
+#pragma unroll
+            for (int a = 0; a < NA; a++) gt[run & 1][group][d][a][lane] = r[a];
+        }
+        asm volatile("bar.sync %0, 96;" ::"r"(group + 1) : "memory");
+        if (on) {
+#pragma unroll
+            for (int a = 0; a < NA; a++) {
+                if (a % 3 != d) continue;
+                double gs = 0.0;
+#pragma unroll
+                for (int i = 0; i < 3; i++) gs = fma(gt[run & 1][group][i][a][lane], LatR<double>::gfac(L, i), gs);
+                if (rho) {
+                    const double r = __ldg(rho + (I)a * (I)L.V + s);
+                    gs -= r;
+                    p[4] = fma(r, r, p[4]);
+                }
+                p[3] = fma(gs, gs, p[3]);
+            }
+        }
+        if ((++run & 31) == 0) {
+#pragma unroll
+            for (int q = 0; q < 5; q++) { two_sum_add(acc[q], p[q]); p[q] = 0.0; }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+        const double v = warp_sum((acc[q].s + p[q]) + acc[q].c);
+        if (lane == 0) sh[q][group * 3 + d] = v;
+    }
+    __syncthreads();
+    for (int q = (int)(threadIdx.x >> 5); q < NQS; q += 3 * G) {
+        // columns 6 and 7: every warp's; the others: those of one direction
+        const int kind = q < 3 ? 0 : (q < 6 ? 1 : (q < 8 ? q - 3 : 2)), i = q < 6 ? q % 3 : q - 8;
+        const bool mine = lane < 3 * G && (q == 6 || q == 7 || lane % 3 == i);
+        double v = warp_sum(mine ? sh[kind][lane] : 0.0);
+        if (lane == 0) {
+            if (q != 6 && q != 7) v *= (q < 3 ? 1.0 : 0.5) * (i == 0 ? L.ufac[0] : (i == 1 ? L.ufac[1] : L.ufac[2]));
+            part[((long)blockIdx.x * NQS + q) * 2] = v;
+            part[((long)blockIdx.x * NQS + q) * 2 + 1] = 0.0;
+        }
+    }
+    last_block_combine<NQS>(part, count, out);
+}
+
+// blocks whose partials the handle's buffer holds: 32 sites each at least, 1216 at most
+int bulk_blocks_max(long V) { return (int)std::min<long>(grid_for(V, 32), 8L * 152); }
 int reduction_blocks(long V) { return (int)std::min<long>(grid_for(V, RED_THREADS), 8L * 152); }
 
 // SU(3) FP32: two sites per thread in paired FP32 instructions (the
@@ -292,16 +389,34 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
 // Blocks of one kernel resident on the whole device at once: the grid-stride
 // reductions then run in a single wave with equal work per thread.
 template <typename K>
-static int resident_blocks(K kernel) {
+static int resident_blocks(K kernel, int threads = RED_THREADS) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RED_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
     return std::max(1, per_sm) * std::max(1, sms);
+}
+
+template <int NC, typename I>
+static void bulk_fx(Ctx &c, int skip_u) {
+    constexpr int T = BulkFx<NC>::groups * 96;
+    static const int wave = resident_blocks(k_bulk_partial_fx<NC, I>, T);
+    const long want = (c.L.V + BulkFx<NC>::groups * 32 - 1) / (BulkFx<NC>::groups * 32);
+    const int nb = (int)std::min<long>(std::min(bulk_blocks_max(c.L.V), wave), want);
+    ensure_fixed_links(c, true, true);
+    k_bulk_partial_fx<NC, I><<<nb, T, 0, c.stream>>>(
+        (const int2 *)c.fx_U, (const int2 *)c.fx_Unext, (const double *)c.U, (const double *)c.Unext, (const double *)c.E,
+        (const double *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L, skip_u, c.red_part, c.red_count, c.red_out, c.bn_site);
+    c.launches += 1;
 }
 
 template <int NC, typename R>
 static void bulk_t(Ctx &c, int skip_u) {
+    if (sizeof(R) == 8 && c.fixed_kernel) {
+        if (c.int_offsets) bulk_fx<NC, int>(c, skip_u);
+        else bulk_fx<NC, long>(c, skip_u);
+        return;
+    }
     int nb = c.red_blocks;
     if (NC == 3 && sizeof(R) == 4 && c.pair_kernel) {
         if (c.int_offsets) {
@@ -365,81 +480,99 @@ __global__ void k_energy_density(const R *__restrict__ U, const R *__restrict__ 
     out[s] = en;
 }
 
-// Block (k, part) sums slice x_dir = k over its share of the transverse sites;
-// six sums per block (PROJ_COLUMNS): T_el, T_mag of U, L_el, L_mag of U, T_mag
+// Block (k, part) sums slice x_dir = k over its share of the transverse sites:
+// per direction j the sums of E_j^2, |B_j(U)|^2 and |B_j(Unext)|^2, and from them
+// six per block (PROJ_COLUMNS): T_el, T_mag of U, L_el, L_mag of U, T_mag
 // of Unext, L_mag of Unext, combined per slice in a fixed order by
 // k_projected_final.  The magnetic sums of U and Unext stay apart so that a
 // call after one step can take U's from the previous call's Unext (skip_u).
+// FP64-pipe bound: the unit factors (g a_j)^-2 are applied to the block's sums, not
+// to every term (two FP64 divisions a term took three quarters of the kernel:
+// 256 x 64^2 SU(2) FP64 in a run with a reduction before each call 0.303 -> 0.104 ms), and the site comes from
+// multiplications and shifts.
 constexpr int PROJ_COLUMNS = 6;
 template <int NC, typename R>
 __global__ void __launch_bounds__(RED_THREADS, RedBounds<NC, R>::minb)
     k_projected_energy(const R *__restrict__ U, const R *__restrict__ Unext, const R *__restrict__ E,
                        const uint8_t *__restrict__ eval, Lat L, int dir, int skip_u,
-                       const double *__restrict__ bn_site, double *__restrict__ part) {
+                       const double *__restrict__ bn_site, const int2 *__restrict__ Uf, const int2 *__restrict__ Unf,
+                       double *__restrict__ part) {
     using G = typename GroupOf<NC, R>::T;
     constexpr int NA = G::NA;
     const LinkPlanes<G, R> Up{const_cast<R *>(U), L.V}, Unp{const_cast<R *>(Unext), L.V};
     const AlgPlanes<NA, R> Ep{const_cast<R *>(E), L.V};
+    __shared__ double ws[9][RED_THREADS / 32];
     const int k = blockIdx.x, nsplit = gridDim.y;
-    const int o1 = (dir + 1) % 3, o2 = (dir + 2) % 3;
-    const long nt = L.V / L.n[dir];
-    const double area = (double)L.V / (double)L.n[dir];
+    // the slower and the faster of the slice's two directions
+    const int hi = dir == 0 ? 1 : 0, lo = dir == 2 ? 1 : 2;
+    const int nlo = lo == 2 ? L.n[2] : L.n[1], nt = (int)(L.V / pick(L.n[0], L.n[1], L.n[2], dir));
     // a thread's sites of the slice are summed plainly in FP64 (a handful per
-    // thread: nt / (nsplit * blockDim) of them), the block's threads with
+    // thread: nt / (nsplit * blockDim) of them), the block's warps with
     // compensation; the FP64 pipe is narrow on this part
-    double p[PROJ_COLUMNS];
+    double p[9];  // E_j^2, B_j(U)^2, B_j(Unext)^2
 #pragma unroll
-    for (int q = 0; q < PROJ_COLUMNS; q++) p[q] = 0.0;
-    for (long t = (long)blockIdx.y * blockDim.x + threadIdx.x; t < nt; t += (long)nsplit * blockDim.x) {
+    for (int q = 0; q < 9; q++) p[q] = 0.0;
+    for (int t = (int)(blockIdx.y * blockDim.x + threadIdx.x); t < nt; t += nsplit * (int)blockDim.x) {
         int x[3];
-        x[dir] = k;
-        const int lo = (o1 > o2) ? o1 : o2, hi = (o1 > o2) ? o2 : o1;  // hi = slower of the two
-        x[lo] = (int)(t % L.n[lo]);
-        x[hi] = (int)(t / L.n[lo]);
+        const int h = div_n(L, lo == 2 ? 0 : 1, t), l = t - h * nlo;
+        x[0] = dir == 0 ? k : h;
+        x[1] = dir == 1 ? k : (hi == 1 ? h : l);
+        x[2] = dir == 2 ? k : l;
         const long s = x[0] * L.stride[0] + x[1] * L.stride[1] + x[2];
         if (eval && !eval[s]) continue;
         const Nbr nb = neighbours(L, s, x);
-        double el_t = 0, el_l = 0, mu_t = 0, mu_l = 0, mn_t = 0, mn_l = 0;
-#pragma unroll 1
+#pragma unroll
         for (int j = 0; j < 3; j++) {
-            const double uf = 1.0 / ((L.g * L.a[j]) * (L.g * L.a[j])) / area;
             R e[NA], b0[NA], b1[NA];
             Ep.load_ro(j, s, e);
-            double mu = 0.0;
+            p[j] += sqr<R, NA>(e);
+            if constexpr (sizeof(R) == 8) {
+                // the values of the BulkQuantities pass (bn_site) bit for bit
+                if (Uf) {
+                    const Deltas<long> D = deltas<long>(L, x);
+                    if (!skip_u) p[3 + j] += fx::plane_b2<long>(fx::FxLinks<NC, long>{Uf, L.V}, U, L, s, x, D, j);
+                    p[6 + j] += bn_site ? __ldg(bn_site + (long)j * L.V + s)
+                                        : fx::plane_b2<long>(fx::FxLinks<NC, long>{Unf, L.V}, Unext, L, s, x, D, j);
+                    continue;
+                }
+            }
             if (!skip_u) {
                 field_b<G, R>(Up, L, s, nb, j, b0);
-                mu = 0.25 * sqr<R, NA>(b0) * uf;
+                p[3 + j] += sqr<R, NA>(b0);
             }
-            double bn;
             if (bn_site) {
-                bn = __ldg(bn_site + (long)j * L.V + s);
+                p[6 + j] += __ldg(bn_site + (long)j * L.V + s);
             } else {
                 field_b<G, R>(Unp, L, s, nb, j, b1);
-                bn = sqr<R, NA>(b1);
+                p[6 + j] += sqr<R, NA>(b1);
             }
-            const double el = 0.5 * sqr<R, NA>(e) * uf;
-            const double mn = 0.25 * bn * uf;
-            if (j == dir) { el_l += el; mu_l += mu; mn_l += mn; } else { el_t += el; mu_t += mu; mn_t += mn; }
-        }
-        p[0] += el_t;
-        p[2] += el_l;
-        p[4] += mn_t;
-        p[5] += mn_l;
-        if (!skip_u) {
-            p[1] += mu_t;
-            p[3] += mu_l;
         }
     }
-    KSum acc[PROJ_COLUMNS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < PROJ_COLUMNS; q++) acc[q] = KSum{p[q], 0.0};
-    int q;
-    KSum v = block_reduce<PROJ_COLUMNS>(acc, q);
-    if (q >= 0) {
-        const long o = (((long)k * nsplit + blockIdx.y) * PROJ_COLUMNS + q) * 2;
-        part[o] = v.s;
-        part[o + 1] = v.c;
+    for (int q = 0; q < 9; q++) {
+        double v = p[q];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) ws[q][warp] = v;
     }
+    __syncthreads();
+    if (threadIdx.x >= PROJ_COLUMNS) return;
+    // column q: electric (0) or magnetic of U (1) or Unext (2); transverse or longitudinal
+    const int q = threadIdx.x, kind = q == 0 || q == 2 ? 0 : (q == 1 || q == 3 ? 1 : 2);
+    const bool longitudinal = q == 2 || q == 3 || q == 5;
+    const double area = (double)L.V / (double)L.n[dir];
+    KSum v{0.0, 0.0};
+    for (int j = 0; j < 3; j++) {
+        if ((j == dir) != longitudinal) continue;
+        KSum c{0.0, 0.0};
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) two_sum_add(c, ws[3 * kind + j][w]);
+        const double f = (kind == 0 ? 0.5 : 0.25) / ((L.g * L.a[j]) * (L.g * L.a[j])) / area;
+        ksum_merge(v, KSum{c.s * f, c.c * f});
+    }
+    const long o = (((long)k * nsplit + blockIdx.y) * PROJ_COLUMNS + q) * 2;
+    part[o] = v.s;
+    part[o + 1] = v.c;
 }
 
 // out[q][k] for the six columns of slice k
@@ -642,8 +775,11 @@ static void projected_energy_t(Ctx &c, int dir, int skip_u, const double *bn_sit
     int nsplit = (int)std::max<long>(1, std::min<long>(c.red_blocks / ns, nt / RED_THREADS));
     nsplit = (int)std::min<long>(nsplit, cap / (2L * PROJ_COLUMNS * ns));
     nsplit = std::max(nsplit, 1);
+    const bool fixed = sizeof(R) == 8 && c.fixed_kernel;
+    if (fixed) ensure_fixed_links(c, !skip_u, !bn_site);
     k_projected_energy<NC, R><<<dim3(ns, nsplit), RED_THREADS, 0, c.stream>>>(
-        (const R *)c.U, (const R *)c.Unext, (const R *)c.E, c.eval, c.L, dir, skip_u, bn_site, c.red_part);
+        (const R *)c.U, (const R *)c.Unext, (const R *)c.E, c.eval, c.L, dir, skip_u, bn_site,
+        fixed ? (const int2 *)c.fx_U : nullptr, fixed ? (const int2 *)c.fx_Unext : nullptr, c.red_part);
     k_projected_final<<<grid_for((long)PROJ_COLUMNS * ns, 128), 128, 0, c.stream>>>(c.red_part, ns, nsplit, out);
     c.launches += 2;
 }

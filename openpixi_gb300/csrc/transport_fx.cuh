@@ -1,0 +1,158 @@
+// transport_fx.cuh -- the parallel transport U^dagger X U of an FP64 algebra
+// element with its group products in fixed point (fixed.cuh), and the Gauss law's
+// term of it.  The element is scaled by a power of two of its largest entry; the
+// transport's error is then below 2^-59 of that entry.  Links that are not
+// usable, or lie within 2^-7 of the identity, and elements that are zero,
+// not finite or near the end of the exponent range take the FP64 products.
+#pragma once
+#include "fixed.cuh"
+
+namespace opx {
+namespace fx {
+
+// Entries of U^dagger X U for X = x_a t_a, x below 2^(k - s) in magnitude, in
+// units of 2^(k - 61): generator components
+template <int NA> struct Scaled {
+    i64 v[NA];
+    double unit;
+};
+// x 2^(e_x - emax - lift) 2^61: the bits of fixed_of below a common exponent
+__device__ __forceinline__ Fx fx_below(double x, int emax, int lift) {
+    const i64 b = bits_of(x);
+    const int e = (int)(b >> 52) & 0x7ff;
+    const uint64_t m = (((uint64_t)b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 10;
+    const unsigned r0 = (unsigned)(lift + emax - e), r = r0 < 63u ? r0 : 63u;
+    const i64 g = (i64)(((m >> r) + 1) >> 1), s = b >> 63;
+    return from_value((g ^ s) - s);
+}
+// x_a below 1/2 (lift 2): U^dagger X U of a pure quaternion
+__device__ __forceinline__ void transport(const Q &U, const double *x, int emax, Scaled<3> &t) {
+    Q X;
+    X.e[0] = Fx{0, 0};
+#pragma unroll
+    for (int a = 0; a < 3; a++) X.e[1 + a] = fx_below(x[a], emax, 2);
+    const Q A = qmul<false, false>(X, U);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        Acc s = acc0v();
+        qcomp<true, false>(s, U, A, 1 + a);
+        t.v[a] = value(s);
+    }
+    t.unit = of_bits((i64)(emax - 59) << 52);  // 2^(emax - 1021 - 61)
+}
+// x_a below 1/4 (lift 3): with 2 X = x_a lambda_a, entries of U^dagger (2 X) U,
+// row by row.  U: the link's entries
+template <class B>
+__device__ __forceinline__ void transport(const B &U, const double *x, int emax, Scaled<8> &t) {
+    const Fx g2 = fx_below(x[2], emax, 3), g7 = fx_below(x[7] * 0.57735026918962576451, emax, 3);
+    const Fx h0 = from_value(to_value(g2) + to_value(g7)), h1 = from_value(to_value(g7) - to_value(g2)), h2 = from_value(-2 * to_value(g7));
+    const Fx ur = fx_below(x[0], emax, 3), vr = fx_below(x[3], emax, 3), wr = fx_below(x[5], emax, 3);
+    const Fx ui = neg(fx_below(x[1], emax, 3)), vi = neg(fx_below(x[4], emax, 3)), wi = neg(fx_below(x[6], emax, 3));
+    // the hermitian matrix's entries: upper 01, 02, 12 = u, v, w, the lower ones conjugate
+    auto H = [&](int c, Fx &re, Fx &im) {
+        const Fx zero{0, 0};
+        switch (c) {
+        case 0: re = h0; im = zero; break;
+        case 1: re = ur; im = ui; break;
+        case 2: re = vr; im = vi; break;
+        case 3: re = ur; im = neg(ui); break;
+        case 4: re = h1; im = zero; break;
+        case 5: re = wr; im = wi; break;
+        case 6: re = vr; im = neg(vi); break;
+        case 7: re = wr; im = neg(wi); break;
+        default: re = h2; im = zero; break;
+        }
+    };
+    i64 w0 = 0, w1 = 0, w2 = 0;
+#pragma unroll 1
+    for (int r = 0; r < 3; r++) {
+        // row r of U^dagger H U, r = 0: entries 00, 01, 02; r = 1: 11, 12; r = 2: 22
+        const Row v = rmul<false>(U.adj_row(r), H);
+        i64 re[3], im[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            Acc a = acc0v(), b = acc0v();
+            rterm<false>(a, b, v, U, q);
+            re[q] = value(a);
+            im[q] = value(b);
+        }
+        if (r == 0) {
+            w0 = re[0];
+            t.v[0] = re[1];
+            t.v[1] = -im[1];
+            t.v[3] = re[2];
+            t.v[4] = -im[2];
+        } else if (r == 1) {
+            w1 = re[1];
+            t.v[5] = re[2];
+            t.v[6] = -im[2];
+        } else {
+            w2 = re[2];
+        }
+    }
+    t.v[2] = (w0 - w1) >> 1;
+    t.v[7] = ((w0 + w1) >> 1) - w2;  // x sqrt 3
+    t.unit = of_bits((i64)(emax - 58) << 52);
+}
+__device__ __forceinline__ double component(const Scaled<3> &t, int a) { return (double)t.v[a]; }
+__device__ __forceinline__ double component(const Scaled<8> &t, int a) {
+    return a == 7 ? (double)t.v[7] * 0.57735026918962576451 : (double)t.v[a];
+}
+
+template <int NC>
+__device__ __forceinline__ void transport_f64(const double *__restrict__ U, const Lat &L, long s, int i, const double *x, double *t) {
+    using G = typename GroupOf<NC, double>::T;
+    const LinkPlanes<G, double> Up{const_cast<double *>(U), L.V};
+    G::act(x, G::adj(Up.load(i, s)), t);
+}
+
+// Whether a link's transport is formed in fixed point
+template <class T> __device__ __forceinline__ bool transportable(const T &u) { return first(u).h != LINK_BAD && offdiag(u) >= WEAK_H; }
+// the entries of a link held in registers
+struct HeldEntries {
+    const M &m;
+    __device__ __forceinline__ void operator()(int c, Fx &re, Fx &im) const {
+        re = m.r[c];
+        im = m.i[c];
+    }
+    __device__ __forceinline__ Row adj_row(int r) const {
+        Row v;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const Fx re = r == 0 ? m.r[3 * k] : (r == 1 ? m.r[3 * k + 1] : m.r[3 * k + 2]);
+            const Fx im = r == 0 ? m.i[3 * k] : (r == 1 ? m.i[3 * k + 1] : m.i[3 * k + 2]);
+            v.r[k] = re;
+            v.i[k] = neg(im);
+        }
+        return v;
+    }
+};
+
+// r = E_i(x) - U_i(x-i)^dagger E_i(x-i) U_i(x-i), sm = x - i, Ub = U_i(x-i) in
+// fixed point (SU(3): its entries), fixed: whether to use it
+template <int NC, typename I, class T>
+__device__ __forceinline__ void gauss_term(const T &Ub, bool fixed, const double *__restrict__ U,
+                                           const double *__restrict__ E, const Lat &L, I s, I sm, int i, double *r) {
+    constexpr int NA = NC == 2 ? 3 : 8;
+    const AlgPlanes<NA, double, I> Ep{const_cast<double *>(E), (I)L.V};
+    double e0[NA], e1[NA];
+    Ep.load_ro(i, s, e0);
+    Ep.load_ro(i, sm, e1);
+    int emax = 0;
+#pragma unroll
+    for (int a = 0; a < NA; a++) { const int e = exponent_of(e1[a]); emax = e > emax ? e : emax; }
+    if (fixed && emax >= 64 && emax < 0x7ff) {
+        Scaled<NA> t;
+        transport(Ub, e1, emax, t);
+#pragma unroll
+        for (int a = 0; a < NA; a++) r[a] = fma(-component(t, a), t.unit, e0[a]);
+    } else {
+        double t[NA];
+        transport_f64<NC>(U, L, (long)sm, i, e1, t);
+#pragma unroll
+        for (int a = 0; a < NA; a++) r[a] = e0[a] - t[a];
+    }
+}
+
+}  // namespace fx
+}  // namespace opx
