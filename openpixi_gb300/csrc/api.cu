@@ -138,7 +138,8 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     c.int_offsets = std::getenv("OPX_LONG_OFFSETS") == nullptr && link_elems(V, c.ng) < (1L << 31) - 64 &&
                     3L * c.na * V < (1L << 31);
     c.rsize = c.prec == OPX_F64 ? 8 : 4;
-    c.fixed_kernel = c.prec == OPX_F64 && std::getenv("OPX_FP64_ONLY") == nullptr && c.L.inva2[0] == c.L.inva2[1] &&
+    c.fp64_only = std::getenv("OPX_FP64_ONLY") != nullptr;
+    c.fixed_kernel = c.prec == OPX_F64 && !c.fp64_only && c.L.inva2[0] == c.L.inva2[1] &&
                      c.L.inva2[1] == c.L.inva2[2];
     bool ok = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) == cudaSuccess;
     auto al = [&](void **p, size_t bytes) { if (ok && cudaMalloc(p, bytes) != cudaSuccess) { ok = false; *p = nullptr; } };

@@ -458,8 +458,8 @@ void ensure_fixed_links(Ctx &c, bool u, bool unext) {
     const dim3 grid(grid_for(c.L.V, 128), 3);
     auto fill = [&](const void *links, void *out, bool &ok) {
         if (ok) return;
-        if (c.nc == 2) fx::k_fixed_links<2><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
-        else fx::k_fixed_links<3><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
+        if (c.nc == 2) fx::k_fixed_links<2, double><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
+        else fx::k_fixed_links<3, double><<<grid, 128, 0, c.stream>>>((const double *)links, (int2 *)out, c.L);
         c.launches++;
         ok = true;
     };

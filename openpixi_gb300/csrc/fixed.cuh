@@ -565,19 +565,22 @@ template <typename I> struct FxLinks<3, I> {
     }
 };
 
-// Link (d, s) of U in fixed point into out
-template <int NC, typename I>
-__device__ __forceinline__ void fixed_link(const double *U, int2 *out, I V, int d, I s) {
+// Link (d, s) of U (double, or float: widened) in fixed point into out
+template <int NC, typename R, typename I>
+__device__ __forceinline__ void fixed_link(const R *U, int2 *out, I V, int d, I s) {
     constexpr int NG = LinkOf<NC>::NG;
     double u[NG];
     const I o = link_offset_t<I>(V, NG, d, 0, s);
-    if constexpr (NC == 2) {
+    if constexpr (NC == 2 && sizeof(R) == 8) {
         const double2 *b = reinterpret_cast<const double2 *>(U + o);
         const double2 x = b[0], y = b[1];
         u[0] = x.x; u[1] = x.y; u[2] = y.x; u[3] = y.y;
+    } else if constexpr (NC == 2) {
+        const float4 x = *reinterpret_cast<const float4 *>(U + o);
+        u[0] = x.x; u[1] = x.y; u[2] = x.z; u[3] = x.w;
     } else {
 #pragma unroll
-        for (int c = 0; c < NG; c++) u[c] = U[o + 32 * c];
+        for (int c = 0; c < NG; c++) u[c] = (double)U[o + 32 * c];
     }
     auto m = link_of<NC>(u);
     if constexpr (NC == 2) {
@@ -594,10 +597,10 @@ __device__ __forceinline__ void fixed_link(const double *U, int2 *out, I V, int 
 }
 
 // One link per thread (blockIdx.y its direction)
-template <int NC>
-__global__ void __launch_bounds__(128) k_fixed_links(const double *__restrict__ U, int2 *__restrict__ out, Lat L) {
+template <int NC, typename R>
+__global__ void __launch_bounds__(128) k_fixed_links(const R *__restrict__ U, int2 *__restrict__ out, Lat L) {
     const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < L.V) fixed_link<NC, long>(U, out, L.V, (int)blockIdx.y, s);
+    if (s < L.V) fixed_link<NC, R, long>(U, out, L.V, (int)blockIdx.y, s);
 }
 #endif
 

@@ -77,7 +77,7 @@ struct Ctx {
     // Unext in fixed point beside the doubles (swapped with them); fx_*_ok: whether
     // they hold the present links (cleared by every entry point that may write
     // links otherwise than the fixed-point update does)
-    bool fixed_kernel = true;
+    bool fixed_kernel = true, fp64_only = false;
     void *fx_U = nullptr, *fx_Unext = nullptr;
     bool fx_U_ok = false, fx_Unext_ok = false;
     void links_changed() { fx_U_ok = fx_Unext_ok = false; }

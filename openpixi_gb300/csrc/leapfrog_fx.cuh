@@ -281,7 +281,7 @@ k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, dou
     if (!update_link<HAS_J, I>(FxLinks<NC, I>{Uf, (I)L.V}, U, E, J, Unext, L, s, i))
         update_link_f64<NC, HAS_J, I>(U, E, J, Unext, L, s, i);
     // the new link in fixed point, from the double that was stored
-    fixed_link<NC, I>(Unext, Unf, (I)L.V, i, s);
+    fixed_link<NC, double, I>(Unext, Unf, (I)L.V, i, s);
 }
 
 }  // namespace fx

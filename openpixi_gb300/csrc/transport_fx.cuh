@@ -25,24 +25,29 @@ __device__ __forceinline__ Fx fx_below(double x, int emax, int lift) {
     const i64 g = (i64)(((m >> r) + 1) >> 1), s = b >> 63;
     return from_value((g ^ s) - s);
 }
-// x_a below 1/2 (lift 2): U^dagger X U of a pure quaternion
+// x_a below 1/2 (lift 2): U^dagger X U, or (FWD) U X U^dagger, of a pure quaternion
+template <bool FWD = false>
 __device__ __forceinline__ void transport(const Q &U, const double *x, int emax, Scaled<3> &t) {
     Q X;
     X.e[0] = Fx{0, 0};
 #pragma unroll
     for (int a = 0; a < 3; a++) X.e[1 + a] = fx_below(x[a], emax, 2);
-    const Q A = qmul<false, false>(X, U);
+    const Q A = qmul<false, FWD>(X, U);
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         Acc s = acc0v();
-        qcomp<true, false>(s, U, A, 1 + a);
+        qcomp<!FWD, false>(s, U, A, 1 + a);
         t.v[a] = value(s);
     }
     t.unit = of_bits((i64)(emax - 59) << 52);  // 2^(emax - 1021 - 61)
 }
-// x_a below 1/4 (lift 3): with 2 X = x_a lambda_a, entries of U^dagger (2 X) U,
-// row by row.  U: the link's entries
-template <class B>
+template <bool FWD, class B> __device__ __forceinline__ Row start_row(const B &U, int r) {
+    if constexpr (FWD) return U.row(r);
+    else return U.adj_row(r);
+}
+// x_a below 1/4 (lift 3): with 2 X = x_a lambda_a, entries of U^dagger (2 X) U, or
+// (FWD) U (2 X) U^dagger, row by row.  U: the link's entries
+template <bool FWD = false, class B>
 __device__ __forceinline__ void transport(const B &U, const double *x, int emax, Scaled<8> &t) {
     const Fx g2 = fx_below(x[2], emax, 3), g7 = fx_below(x[7] * 0.57735026918962576451, emax, 3);
     const Fx h0 = from_value(to_value(g2) + to_value(g7)), h1 = from_value(to_value(g7) - to_value(g2)), h2 = from_value(-2 * to_value(g7));
@@ -66,13 +71,13 @@ __device__ __forceinline__ void transport(const B &U, const double *x, int emax,
     i64 w0 = 0, w1 = 0, w2 = 0;
 #pragma unroll 1
     for (int r = 0; r < 3; r++) {
-        // row r of U^dagger H U, r = 0: entries 00, 01, 02; r = 1: 11, 12; r = 2: 22
-        const Row v = rmul<false>(U.adj_row(r), H);
+        // row r of the product, r = 0: entries 00, 01, 02; r = 1: 11, 12; r = 2: 22
+        const Row v = rmul<false>(start_row<FWD>(U, r), H);
         i64 re[3], im[3];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             Acc a = acc0v(), b = acc0v();
-            rterm<false>(a, b, v, U, q);
+            rterm<FWD>(a, b, v, U, q);
             re[q] = value(a);
             im[q] = value(b);
         }
@@ -99,11 +104,21 @@ __device__ __forceinline__ double component(const Scaled<8> &t, int a) {
     return a == 7 ? (double)t.v[7] * 0.57735026918962576451 : (double)t.v[a];
 }
 
-template <int NC>
-__device__ __forceinline__ void transport_f64(const double *__restrict__ U, const Lat &L, long s, int i, const double *x, double *t) {
+template <int NC, bool FWD, typename R>
+__device__ __forceinline__ void transport_f64(const R *__restrict__ U, const Lat &L, long s, int i, const double *x, double *t) {
     using G = typename GroupOf<NC, double>::T;
-    const LinkPlanes<G, double> Up{const_cast<double *>(U), L.V};
-    G::act(x, G::adj(Up.load(i, s)), t);
+    using GR = typename GroupOf<NC, R>::T;
+    const auto u = LinkPlanes<GR, R>{const_cast<R *>(U), L.V}.load(i, s);
+    typename G::M g;
+    if constexpr (NC == 2) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) g.e[c] = (double)u.e[c];
+    } else {
+#pragma unroll
+        for (int c = 0; c < 9; c++) { g.r[c] = (double)u.r[c]; g.i[c] = (double)u.i[c]; }
+    }
+    if constexpr (FWD) G::act(x, g, t);
+    else G::act(x, G::adj(g), t);
 }
 
 // Whether a link's transport is formed in fixed point
@@ -128,6 +143,28 @@ struct HeldEntries {
     }
 };
 
+// r = x0 - U^dagger x U, or (FWD) x0 - U x U^dagger, U the link (i, s) of the array U and
+// Uf the same in fixed point (SU(3): its entries), fixed: whether to use that
+template <int NC, bool FWD, typename R, class T>
+__device__ __forceinline__ void minus_transported(const T &Uf, bool fixed, const R *__restrict__ U, const Lat &L, long s, int i,
+                                                  const double *x0, const double *x, double *r) {
+    constexpr int NA = NC == 2 ? 3 : 8;
+    int emax = 0;
+#pragma unroll
+    for (int a = 0; a < NA; a++) { const int e = exponent_of(x[a]); emax = e > emax ? e : emax; }
+    if (fixed && emax >= 64 && emax < 0x7ff) {
+        Scaled<NA> t;
+        transport<FWD>(Uf, x, emax, t);
+#pragma unroll
+        for (int a = 0; a < NA; a++) r[a] = fma(-component(t, a), t.unit, x0[a]);
+    } else {
+        double t[NA];
+        transport_f64<NC, FWD, R>(U, L, s, i, x, t);
+#pragma unroll
+        for (int a = 0; a < NA; a++) r[a] = x0[a] - t[a];
+    }
+}
+
 // r = E_i(x) - U_i(x-i)^dagger E_i(x-i) U_i(x-i), sm = x - i, Ub = U_i(x-i) in
 // fixed point (SU(3): its entries), fixed: whether to use it
 template <int NC, typename I, class T>
@@ -138,20 +175,7 @@ __device__ __forceinline__ void gauss_term(const T &Ub, bool fixed, const double
     double e0[NA], e1[NA];
     Ep.load_ro(i, s, e0);
     Ep.load_ro(i, sm, e1);
-    int emax = 0;
-#pragma unroll
-    for (int a = 0; a < NA; a++) { const int e = exponent_of(e1[a]); emax = e > emax ? e : emax; }
-    if (fixed && emax >= 64 && emax < 0x7ff) {
-        Scaled<NA> t;
-        transport(Ub, e1, emax, t);
-#pragma unroll
-        for (int a = 0; a < NA; a++) r[a] = fma(-component(t, a), t.unit, e0[a]);
-    } else {
-        double t[NA];
-        transport_f64<NC>(U, L, (long)sm, i, e1, t);
-#pragma unroll
-        for (int a = 0; a < NA; a++) r[a] = e0[a] - t[a];
-    }
+    minus_transported<NC, false, double>(Ub, fixed, U, L, (long)sm, i, e0, e1, r);
 }
 
 }  // namespace fx
