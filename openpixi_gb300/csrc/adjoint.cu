@@ -44,11 +44,13 @@
 //       Wbar_i(x) += Mbar S^*,  Sbar = W_i(x)^* Mbar
 //   S = sum_j c_j [A_j + B_j], A = P Q^* R^*, B = P^* Q^* R (Grid.getStapleSum,
 //       Grid.java:675-696), c_j = 1/a_j^2: the cotangents of the staple links
-//       are gathered by each link from the (up to) twelve staples it enters.
+//       are gathered by each link from the (up to) twelve staples it enters
+//       (adjoint_fx.cuh).
 // SU(2) only.
 #include <algorithm>
 #include <vector>
 
+#include "adjoint_fx.cuh"
 #include "dual.cuh"
 #include "internal.h"
 #include "ksum.cuh"
@@ -110,87 +112,42 @@ __device__ __forceinline__ Q staple_sum(const LinkPlanes<G2, double> &W, const L
     return S;
 }
 
-// Pass 1 of the reverse step: per link, the local cotangents.
-__global__ void k_adj_local(const double *__restrict__ Wprev, const double *__restrict__ Enew,
-                            const double *__restrict__ Wbar_new, const double *__restrict__ Ebar_new, Lat L,
-                            double *__restrict__ Sbar, double *__restrict__ Uown, double *__restrict__ Ebar_prev) {
-    const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= L.V) return;
-    const LinkPlanes<G2, double> W{const_cast<double *>(Wprev), L.V}, Wb{const_cast<double *>(Wbar_new), L.V};
-    const LinkPlanes<G2, double> SB{Sbar, L.V}, UO{Uown, L.V};
-    const AlgPlanes<3, double> En{const_cast<double *>(Enew), L.V}, Eb{const_cast<double *>(Ebar_new), L.V};
-    const AlgPlanes<3, double> Ep{Ebar_prev, L.V};
+// Pass 1 of the reverse step: the local cotangents, one link per thread; the staple
+// sum in fixed point beside the FP64 of the rest (64^3: 0.39 -> 0.17 ms).
+template <typename I>
+__global__ void __launch_bounds__(128, 4)
+k_adj_local(const int2 *__restrict__ Wf, const double *__restrict__ Wprev, const double *__restrict__ Enew,
+            const double *__restrict__ Wbar_new, const double *__restrict__ Ebar_new, const __grid_constant__ Lat L, int fixed,
+            double *__restrict__ Mv, double *__restrict__ Uown, double *__restrict__ Ebar_prev) {
+    const unsigned chunk = blockIdx.x / 3u;
+    const int i = (int)(blockIdx.x - 3u * chunk);
+    const I s = (I)chunk * (I)blockDim.x + (I)threadIdx.x;
+    if (s >= (I)L.V) return;
+    const LinkPlanes<G2, double, I> W{const_cast<double *>(Wprev), (I)L.V}, Wb{const_cast<double *>(Wbar_new), (I)L.V};
+    const LinkPlanes<G2, double, I> UO{Uown, (I)L.V};
+    const AlgPlanes<3, double, I> En{const_cast<double *>(Enew), (I)L.V}, Eb{const_cast<double *>(Ebar_new), (I)L.V};
+    const AlgPlanes<3, double, I> Ep{Ebar_prev, (I)L.V}, Mp{Mv, (I)L.V};
     int x[3];
-    site_coords(L, s, x);
+    site_coords<I>(L, s, x);
     const double dt = L.dt;
-    for (int i = 0; i < 3; i++) {
-        const Q Ui = W.load(i, s);
-        double e[3], v[3], eb[3], vb[3];
-        En.load_ro(i, s, e);
-        for (int a = 0; a < 3; a++) v[a] = -dt * e[a];
-        const Q X = G2::expi(v);
-        const Q Wn_b = Wb.load(i, s);
-        Q own = qmul(qadj(X), Wn_b);
-        expi_adjoint(v, qmul(Wn_b, qadj(Ui)), vb);
-        Eb.load_ro(i, s, eb);
-        for (int a = 0; a < 3; a++) eb[a] += -dt * vb[a];
-        const Q Mb{{0.0, 2 * dt * eb[0], 2 * dt * eb[1], 2 * dt * eb[2]}};
-        const Q S = staple_sum(W, L, s, x, i);
-        qacc(own, qmul(Mb, qadj(S)));
-        SB.store(i, s, qmul(qadj(Ui), Mb));
-        UO.store(i, s, own);
-        Ep.store(i, s, eb);
-    }
-}
-
-// Pass 2: each link gathers the cotangents from the staples it belongs to.
-__global__ void k_adj_gather(const double *__restrict__ Wprev, const double *__restrict__ Sbar,
-                             const double *__restrict__ Uown, Lat L, double *__restrict__ Wbar_prev) {
-    const long y = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= L.V) return;
-    const LinkPlanes<G2, double> W{const_cast<double *>(Wprev), L.V}, SB{const_cast<double *>(Sbar), L.V};
-    const LinkPlanes<G2, double> UO{const_cast<double *>(Uown), L.V}, OUT{Wbar_prev, L.V};
-    int x[3];
-    site_coords(L, y, x);
-    for (int k = 0; k < 3; k++) {
-        Q acc = UO.load(k, y);
-        const int xk = pick(x[0], x[1], x[2], k);
-        const long y_pk = shift_d(L, y, xk, k, +1);
-        const double ck = LatR<double>::inva2(L, k);
-        for (int ii = 1; ii < 3; ii++) {
-            const int i = (k + ii) % 3;  // the other direction (i for the A/B-term P,R roles; j for Q roles)
-            const int xi = pick(x[0], x[1], x[2], i);
-            const long y_mi = shift_d(L, y, xi, i, -1);
-            const long y_pi = shift_d(L, y, xi, i, +1);
-            const long y_mi_pk = shift_d(L, y_mi, xk, k, +1);
-            const long y_pk_pi = shift_d(L, y_pk, xi, i, +1);  // unused placeholder for symmetry
-            (void)y_pk_pi;
-            const double ci = LatR<double>::inva2(L, i);
-            // A-term, role P: l = (y - i, i), plane k: += c_k Sbar_l U_k(y-i) U_i(y-i+k)
-            qacc(acc, qscale(qmul(qmul(SB.load(i, y_mi), W.load(k, y_mi)), W.load(i, y_mi_pk)), ck));
-            // A-term, role Q: l = (y - j, k), plane j=i: += c_j (U_j(y-j+k)^* Sbar_l U_j(y-j))^*
-            {
-                const Q P = W.load(i, y_mi_pk), R = W.load(i, y_mi);
-                qacc(acc, qscale(qadj(qmul(qmul(qadj(P), SB.load(k, y_mi)), R)), ci));
-            }
-            // A-term, role R: l = (y, i), plane k: += c_k (U_i(y+k) U_k(y+i)^* Sbar_l)^*
-            {
-                const Q Qv = W.load(i, y_pk), P = W.load(k, y_pi);
-                qacc(acc, qscale(qadj(qmul(qmul(Qv, qadj(P)), SB.load(i, y))), ck));
-            }
-            // B-term, role P: l = (y - i + k, i), plane k: += c_k (Sbar_l U_k(y-i)^* U_i(y-i))^*
-            qacc(acc, qscale(qadj(qmul(qmul(SB.load(i, y_mi_pk), qadj(W.load(k, y_mi))), W.load(i, y_mi))), ck));
-            // B-term, role Q: l = (y + j, k), plane j=i: += c_j (U_j(y+k) Sbar_l U_j(y)^*)^*
-            {
-                const long y_pj = y_pi;
-                const Q P = W.load(i, y_pk), R = W.load(i, y);
-                qacc(acc, qscale(qadj(qmul(qmul(P, SB.load(k, y_pj)), qadj(R))), ci));
-            }
-            // B-term, role R: l = (y + k, i), plane k: += c_k U_i(y) U_k(y+i) Sbar_l
-            qacc(acc, qscale(qmul(qmul(W.load(i, y), W.load(k, y_pi)), SB.load(i, y_pk)), ck));
-        }
-        OUT.store(k, y, acc);
-    }
+    const Q Ui = W.load(i, s);
+    double e[3], v[3], eb[3], vb[3];
+    En.load_ro(i, s, e);
+    for (int a = 0; a < 3; a++) v[a] = -dt * e[a];
+    const Q X = G2::expi(v);
+    const Q Wn_b = Wb.load(i, s);
+    Q own = qmul(qadj(X), Wn_b);
+    expi_adjoint(v, qmul(Wn_b, qadj(Ui)), vb);
+    Eb.load_ro(i, s, eb);
+    for (int a = 0; a < 3; a++) eb[a] += -dt * vb[a];
+    const double m[3] = {2 * dt * eb[0], 2 * dt * eb[1], 2 * dt * eb[2]};
+    Q S;
+    if (!(fixed && fx::staple_sum_fx<I>(fx::FxLinks<2, I>{Wf, (I)L.V}, L, s, deltas<I>(L, x), i, S)))
+        S = staple_sum(LinkPlanes<G2, double>{const_cast<double *>(Wprev), L.V}, L, (long)s, x, i);
+    qacc(own, fx::left_mul(m, qadj(S)));
+    Mp.store(i, s, m);
+    UO.store(i, s, own);
+    Ep.store(i, s, eb);
 }
 
 __device__ __forceinline__ void atomic_add_link(double *base, long V, int d, long s, const Q &q) {
@@ -350,11 +307,14 @@ __global__ void k_obj_box(const R *__restrict__ Wm, const R *__restrict__ Wn, co
     if (q >= 0) { part[2 * (blockIdx.x * 4 + q)] = v.s; part[2 * (blockIdx.x * 4 + q) + 1] = v.c; }
 }
 
-__global__ void k_obj_box_final(const double *__restrict__ part, int nb, double *__restrict__ out) {
-    if (threadIdx.x >= 4) return;
+// warp q sums column q over the blocks: the lanes' shares in order, then the lanes in a
+// compensated tree (tangents may be negative)
+__global__ void __launch_bounds__(128) k_obj_box_final(const double *__restrict__ part, int nb, double *__restrict__ out) {
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
     KSum v{0.0, 0.0};
-    for (int b = 0; b < nb; b++) ksum_merge(v, KSum{part[2 * (b * 4 + threadIdx.x)], part[2 * (b * 4 + threadIdx.x) + 1]});
-    out[threadIdx.x] = v.s + v.c;
+    for (int b = lane; b < nb; b += 32) ksum_merge(v, KSum{part[2 * (b * 4 + q)], part[2 * (b * 4 + q) + 1]});
+    for (int o = 16; o > 0; o >>= 1) ksum_merge(v, KSum{__shfl_down_sync(0xffffffffu, v.s, o), __shfl_down_sync(0xffffffffu, v.c, o)});
+    if (lane == 0) out[q] = v.s + v.c;
 }
 
 // Cotangents of the anisotropy J = A / B with respect to E_N, W_{N-1} and W_N:
@@ -436,8 +396,11 @@ using namespace opx;
 
 namespace {
 
+// Device buffers of one call: get() hands out offsets, take() makes the one
+// allocation and at() the pointers (a gradient's fifty allocations and frees took 3 ms)
 struct DevBuf {
-    std::vector<void *> ptrs;
+    char *base = nullptr;
+    size_t bytes = 0;
     bool ok = true;
     template <typename T> T *get(size_t n) {
         void *p = nullptr;
@@ -445,7 +408,23 @@ struct DevBuf {
         ptrs.push_back(p);
         return (T *)p;
     }
-    ~DevBuf() { for (void *p : ptrs) cudaFree(p); }
+    size_t reserve(size_t n) {
+        const size_t o = bytes;
+        bytes += (n + 255) & ~size_t(255);
+        return o;
+    }
+    bool take() {
+        if (cudaMalloc((void **)&base, std::max<size_t>(bytes, 256)) != cudaSuccess) { ok = false; base = nullptr; cudaGetLastError(); }
+        return ok;
+    }
+    template <typename T> T *at(size_t o) const { return (T *)(base + o); }
+    ~DevBuf() {
+        for (void *p : ptrs) cudaFree(p);
+        if (base) cudaFree(base);
+    }
+
+private:
+    std::vector<void *> ptrs;
 };
 
 struct ObjArgs {
@@ -489,7 +468,7 @@ double objective_value(Ctx &c, const R *Wm, const R *Wn, const R *E, const Obj &
                        double *dJ, double *A_B = nullptr) {
     const int nb = 304;
     k_obj_box<R><<<nb, 256, 0, c.stream>>>(Wm, Wn, E, c.L, ob, part);
-    k_obj_box_final<<<1, 32, 0, c.stream>>>(part, nb, out4);
+    k_obj_box_final<<<1, 128, 0, c.stream>>>(part, nb, out4);
     c.launches += 2;
     double h[4] = {0, 0, 0, 0};
     cudaMemcpyAsync(h, out4, 4 * sizeof(double), cudaMemcpyDeviceToHost, c.stream);
@@ -612,44 +591,69 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
         return OPX_ERR_INVALID;
     }
     const int nseg = (nsteps + ckpt - 1) / ckpt;
-    const int rs = c.prec == OPX_F64 ? 8 : 4;
+    const bool f64 = c.prec == OPX_F64;
+    const int rs = f64 ? 8 : 4;
+    // strides in bytes, whole lines (E's 72 V bytes alone would misalign the links after them)
+    const size_t bU = (size_t)nU * 8, bE = ((size_t)nE * 8 + 255) & ~size_t(255);
+    const int fixed = !c.fp64_only && c.L.inva2[0] == c.L.inva2[1] && c.L.inva2[1] == c.L.inva2[2];
     DevBuf B;
-    // forward in the handle's precision
-    char *Ur0 = B.get<char>(nU * rs), *Wra = B.get<char>(nU * rs), *Wrb = B.get<char>(nU * rs), *Er = B.get<char>(nE * rs);
-    double *U64 = B.get<double>(nU), *E64 = B.get<double>(nE);
-    std::vector<double *> ckW(nseg), ckE(nseg);
-    for (int k = 0; k < nseg; k++) { ckW[k] = B.get<double>(nU); ckE[k] = B.get<double>(nE); }
-    std::vector<double *> segW(ckpt + 1), segE(ckpt + 1);
-    for (int m = 0; m <= ckpt; m++) { segW[m] = B.get<double>(nU); segE[m] = B.get<double>(nE); }
-    double *Wbar[2] = {B.get<double>(nU), B.get<double>(nU)}, *Ebar[2] = {B.get<double>(nE), B.get<double>(nE)};
-    double *Wm_b = B.get<double>(nU), *Sbar = B.get<double>(nU), *Uown = B.get<double>(nU);
-    double *part = B.get<double>(8 * 304), *out4 = B.get<double>(4);
-    if (!B.ok) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
-    cudaMemcpyAsync(Ur0, c.U, nU * rs, cudaMemcpyDeviceToDevice, c.stream);
-    cudaMemcpyAsync(Er, c.E, nE * rs, cudaMemcpyDeviceToDevice, c.stream);
+    // forward in the handle's precision, its links in fixed point beside them (FP64)
+    const size_t oWra = B.reserve(nU * rs), oWrb = B.reserve(nU * rs), oEr = B.reserve(nE * rs), oFa = B.reserve(bU), oFb = B.reserve(bU);
+    const size_t oU64 = B.reserve(bU), oE64 = B.reserve(bE), oCk = B.reserve(nseg * (bU + bE)), oSeg = B.reserve((size_t)ckpt * (2 * bU + bE));
+    const size_t oBar = B.reserve(2 * (bU + bE)), oWm = B.reserve(bU), oM = B.reserve(bE), oUown = B.reserve(bU);
+    const size_t oPart = B.reserve(8 * 8 * 304), oOut = B.reserve(32);
+    if (!B.take()) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
+    double *U64 = B.at<double>(oU64), *E64 = B.at<double>(oE64), *part = B.at<double>(oPart), *out4 = B.at<double>(oOut);
+    double *Wm_b = B.at<double>(oWm), *Mv = B.at<double>(oM), *Uown = B.at<double>(oUown);
+    double *Wbar[2] = {B.at<double>(oBar), B.at<double>(oBar + bU)}, *Ebar[2] = {B.at<double>(oBar + 2 * bU), B.at<double>(oBar + 2 * bU + bE)};
+    char *Er = B.at<char>(oEr);
+    auto ckW = [&](int k) { return B.at<double>(oCk + k * (bU + bE)); };
+    auto ckE = [&](int k) { return B.at<double>(oCk + k * (bU + bE) + bU); };
+    // W_{start + m} and E_{start + m} (m = 1 .. ckpt) of a segment, and the fixed-point form of W_{start + m - 1}
+    auto segW = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * (2 * bU + bE)); };
+    auto segE = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * (2 * bU + bE) + bU); };
+    auto segF = [&](int m) { return B.at<int2>(oSeg + (size_t)(m - 1) * (2 * bU + bE) + bU + bE); };
     widen_state(c, U64, E64);
+    cudaMemcpyAsync(Er, c.E, nE * rs, cudaMemcpyDeviceToDevice, c.stream);
     const dim3 gs(grid_for(V, 128));
+    // one FP64 step from W (fixed point F) with E in place; Fn: W_{n+1} in fixed point
+    auto to_fixed = [&](const double *W, int2 *F) {
+        fx::k_fixed_links<2, double><<<dim3(gs.x, 3), 128, 0, c.stream>>>(W, F, c.L);
+        c.launches++;
+    };
+    auto step64 = [&](const int2 *F, const double *W, double *E, double *Wn, int2 *Fn) {
+        if (!fixed) k_step_plain<2, double, false><<<gs, 128, 0, c.stream>>>(W, E, Wn, c.L);
+        else if (c.int_offsets) fx::k_update_links_fx<2, false, int><<<3 * gs.x, 128, 0, c.stream>>>(F, W, E, nullptr, Wn, Fn, nullptr, c.L);
+        else fx::k_update_links_fx<2, false, long><<<3 * gs.x, 128, 0, c.stream>>>(F, W, E, nullptr, Wn, Fn, nullptr, c.L);
+        c.launches++;
+    };
     auto store_ckpt = [&](int k, char *W) {
-        if (c.prec == OPX_F64) {
-            cudaMemcpyAsync(ckW[k], W, nU * 8, cudaMemcpyDeviceToDevice, c.stream);
-            cudaMemcpyAsync(ckE[k], Er, nE * 8, cudaMemcpyDeviceToDevice, c.stream);
+        if (f64) {
+            cudaMemcpyAsync(ckW(k), W, nU * 8, cudaMemcpyDeviceToDevice, c.stream);
+            cudaMemcpyAsync(ckE(k), Er, nE * 8, cudaMemcpyDeviceToDevice, c.stream);
         } else {
-            k_widen<<<grid_for(nU, 256), 256, 0, c.stream>>>((const float *)W, ckW[k], nU);
-            k_widen<<<grid_for(nE, 256), 256, 0, c.stream>>>((const float *)Er, ckE[k], nE);
+            k_widen<<<grid_for(nU, 256), 256, 0, c.stream>>>((const float *)W, ckW(k), nU);
+            k_widen<<<grid_for(nE, 256), 256, 0, c.stream>>>((const float *)Er, ckE(k), nE);
             c.launches += 2;
         }
     };
-    char *cur = Wra, *nxt = Wrb;
-    if (c.prec == OPX_F64) k_links_plain<2, double><<<gs, 128, 0, c.stream>>>((double *)Ur0, (double *)Er, (double *)cur, c.L);
-    else k_links_plain<2, float><<<gs, 128, 0, c.stream>>>((float *)Ur0, (float *)Er, (float *)cur, c.L);
+    char *cur = B.at<char>(oWra), *nxt = B.at<char>(oWrb);
+    int2 *Fc = B.at<int2>(oFa), *Fn = B.at<int2>(oFb);
+    if (f64) k_links_plain<2, double><<<gs, 128, 0, c.stream>>>((const double *)c.U, (double *)Er, (double *)cur, c.L);
+    else k_links_plain<2, float><<<gs, 128, 0, c.stream>>>((const float *)c.U, (float *)Er, (float *)cur, c.L);
     c.launches++;
     store_ckpt(0, cur);
+    if (f64 && fixed) to_fixed((const double *)cur, Fc);
     for (int n = 1; n < nsteps; n++) {
-        const bool reunit = c.prec == OPX_F32 && c.cfg.reunit_every > 0 && n % c.cfg.reunit_every == 0;
-        if (c.prec == OPX_F64) k_step_plain<2, double, false><<<gs, 128, 0, c.stream>>>((double *)cur, (double *)Er, (double *)nxt, c.L);
-        else if (reunit) k_step_plain<2, float, true><<<gs, 128, 0, c.stream>>>((float *)cur, (float *)Er, (float *)nxt, c.L);
-        else k_step_plain<2, float, false><<<gs, 128, 0, c.stream>>>((float *)cur, (float *)Er, (float *)nxt, c.L);
-        c.launches++;
+        const bool reunit = !f64 && c.cfg.reunit_every > 0 && n % c.cfg.reunit_every == 0;
+        if (f64) {
+            step64(Fc, (const double *)cur, (double *)Er, (double *)nxt, Fn);
+            std::swap(Fc, Fn);
+        } else {
+            if (reunit) k_step_plain<2, float, true><<<gs, 128, 0, c.stream>>>((float *)cur, (float *)Er, (float *)nxt, c.L);
+            else k_step_plain<2, float, false><<<gs, 128, 0, c.stream>>>((float *)cur, (float *)Er, (float *)nxt, c.L);
+            c.launches++;
+        }
         std::swap(cur, nxt);
         if (n % ckpt == 0) store_ckpt(n / ckpt, cur);
     }
@@ -658,33 +662,36 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
     double Jv = 0.0;
     for (int k = nseg - 1; k >= 0; k--) {
         const int start = k * ckpt, len = std::min(ckpt, nsteps - start);
-        cudaMemcpyAsync(segW[0], ckW[k], nU * 8, cudaMemcpyDeviceToDevice, c.stream);
-        cudaMemcpyAsync(segE[0], ckE[k], nE * 8, cudaMemcpyDeviceToDevice, c.stream);
+        auto W_at = [&](int m) { return m == 0 ? ckW(k) : segW(m); };
+        if (fixed) to_fixed(ckW(k), segF(1));
         for (int m = 1; m <= len; m++) {
-            cudaMemcpyAsync(segE[m], segE[m - 1], nE * 8, cudaMemcpyDeviceToDevice, c.stream);
-            k_step_plain<2, double, false><<<gs, 128, 0, c.stream>>>(segW[m - 1], segE[m], segW[m], c.L);
-            c.launches++;
+            cudaMemcpyAsync(segE(m), m == 1 ? ckE(k) : segE(m - 1), nE * 8, cudaMemcpyDeviceToDevice, c.stream);
+            step64(segF(m), W_at(m - 1), segE(m), segW(m), m < len ? segF(m + 1) : Fc);
         }
         if (k == nseg - 1) {
             double AB[2];
-            Jv = objective_value<double>(c, segW[len - 1], segW[len], segE[len], ar.ob, part, out4, nullptr, AB);
+            Jv = objective_value<double>(c, W_at(len - 1), segW(len), segE(len), ar.ob, part, out4, nullptr, AB);
             cudaMemsetAsync(Wm_b, 0, nU * 8, c.stream);
             cudaMemsetAsync(Wbar[wb], 0, nU * 8, c.stream);
             if (ar.ob.kind == OPX_OBJ_ENERGY) {
-                k_adj_objective<<<gs, 128, 0, c.stream>>>(segW[len - 1], segW[len], segE[len], c.L, ar.ob.box, Wm_b,
+                k_adj_objective<<<gs, 128, 0, c.stream>>>(W_at(len - 1), segW(len), segE(len), c.L, ar.ob.box, Wm_b,
                                                           Wbar[wb], Ebar[wb]);
             } else {
                 const double wT = 1.0 / AB[1], wL = (-1.0 - Jv) / AB[1];
-                k_adj_aniso<<<gs, 128, 0, c.stream>>>(segW[len - 1], segW[len], segE[len], c.L, ar.ob, wT, wL, Wm_b,
+                k_adj_aniso<<<gs, 128, 0, c.stream>>>(W_at(len - 1), segW(len), segE(len), c.L, ar.ob, wT, wL, Wm_b,
                                                       Wbar[wb], Ebar[wb]);
             }
             c.launches++;
         }
         for (int m = len; m >= 1; m--) {
             const int n = start + m;
-            k_adj_local<<<gs, 128, 0, c.stream>>>(segW[m - 1], segE[m], Wbar[wb], Ebar[wb], c.L, Sbar, Uown,
-                                                  Ebar[wb ^ 1]);
-            k_adj_gather<<<gs, 128, 0, c.stream>>>(segW[m - 1], Sbar, Uown, c.L, Wbar[wb ^ 1]);
+            if (c.int_offsets) {
+                k_adj_local<int><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), segE(m), Wbar[wb], Ebar[wb], c.L, fixed, Mv, Uown, Ebar[wb ^ 1]);
+                fx::k_adj_gather_fx<int><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), Mv, Uown, c.L, fixed, Wbar[wb ^ 1]);
+            } else {
+                k_adj_local<long><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), segE(m), Wbar[wb], Ebar[wb], c.L, fixed, Mv, Uown, Ebar[wb ^ 1]);
+                fx::k_adj_gather_fx<long><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), Mv, Uown, c.L, fixed, Wbar[wb ^ 1]);
+            }
             c.launches += 2;
             if (n == nsteps) {
                 k_axpy_d<<<grid_for(nU, 256), 256, 0, c.stream>>>(Wbar[wb ^ 1], Wm_b, 1.0, nU);
@@ -696,29 +703,28 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
     // W_0 = exp(-i dt E_0) U
     k_adj_init_links<<<gs, 128, 0, c.stream>>>(U64, E64, Wbar[wb], c.L, Ebar[wb]);
     c.launches++;
-    int rc = finish(c, where);
-    if (rc) return rc;
+    // the gradient in the host's layout (transposed on the device), and to the host
+    Ctx h;  // an FP64 view for the conversion
+    h.L = c.L;
+    h.nc = c.nc;
+    h.na = c.na;
+    h.prec = OPX_F64;
+    h.stream = c.stream;
+    double *dst = Wbar[wb];
     if (wrt == OPX_WRT_E) {
-        std::vector<double> t(nE);
-        cudaMemcpyAsync(t.data(), Ebar[wb], nE * 8, cudaMemcpyDeviceToHost, c.stream);
-        rc = finish(c, where);
-        if (rc) return rc;
-        for (long s = 0; s < V; s++)
-            for (int d = 0; d < 3; d++)
-                for (int a = 0; a < 3; a++) grad[(s * 3 + d) * 3 + a] = t[(d * 3 + a) * V + s];
+        launch_alg_to_host(h, Ebar[wb], dst, 3, OPX_LAYOUT_GEN);
     } else {
         // dJ/drho = K^+ div (dJ/dE_0)
-        double *r = Sbar, *nu = Uown;  // site fields ([3][V]) in the free cotangent buffers
+        double *r = Mv, *nu = Uown;  // site fields ([3][V]) in the free cotangent buffers
         ic_div(c, U64, Ebar[wb], r);
-        rc = ic_covariant_solve(c, U64, r, nu, 1e-13, 20000, nullptr);
+        int rc = ic_covariant_solve(c, U64, r, nu, 1e-13, 20000, nullptr);
         if (rc) { c.err = std::string(where) + ": " + c.err; return rc; }
-        std::vector<double> t(V * 3);
-        cudaMemcpyAsync(t.data(), nu, V * 3 * 8, cudaMemcpyDeviceToHost, c.stream);
-        rc = finish(c, where);
-        if (rc) return rc;
-        for (long s = 0; s < V; s++)
-            for (int a = 0; a < 3; a++) grad[s * 3 + a] = t[a * V + s];
+        launch_alg_to_host(h, nu, dst, 1, OPX_LAYOUT_GEN);
     }
+    c.launches++;
+    cudaMemcpyAsync(grad, dst, want * 8, cudaMemcpyDeviceToHost, c.stream);
+    int rc = finish(c, where);
+    if (rc) return rc;
     *J = Jv;
     return OPX_OK;
 }
