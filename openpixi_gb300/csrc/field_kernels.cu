@@ -83,6 +83,38 @@ k_update_grid_su3f_pair(const float *__restrict__ U, float *__restrict__ E, cons
     update_site_pair<I, HAS_J, REUNIT>(U, E, J, Unext, L, sa, sb, va, vb);
 }
 
+// The same, one link per warp: three consecutive warps share 64 sites.  The work
+// comes in thirds, so a lattice of a few waves fills the last one better and one
+// that does not fill the GPU waits for one link's chain instead of three; a large
+// one loses the own links that the three links of a site share in L1.  ms a step,
+// this form against the other: 24^3 0.0102 / 0.0145, 50 x 45 x 70 0.0392 / 0.0438, 64^3
+// 0.0600 / 0.0662, 96^3 0.185 / 0.189, 128^3 0.438 / 0.425, 192^3 1.48 / 1.43.
+constexpr long LINK_WARPS_MAX_V = 1000000;
+template <typename I, bool HAS_J, bool REUNIT>
+__global__ void __launch_bounds__(128, 3)
+k_update_link_su3f_pair(const float *__restrict__ U, float *__restrict__ E, const float *__restrict__ J,
+                        float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L) {
+    const int lane = threadIdx.x & 31;
+    const unsigned w = blockIdx.x * 4u + (threadIdx.x >> 5);
+    const int i = (int)(w % 3u);
+    const I sa = (I)(w / 3u) * 64 + (I)lane;
+    {
+        const I s0 = sa - (I)lane + (I)((lane & 1) << 5);
+        if (lane < 16 && s0 < (I)L.V) {
+            const float *e = E + (I)(8 * i + (lane >> 1)) * (I)L.V + s0;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(e));
+        }
+    }
+    if (sa >= (I)L.V) return;
+    I sb = sa + 32;
+    bool vb = sb < (I)L.V;
+    if (!vb) sb = sa;
+    const bool va = !active || active[sa];
+    vb = vb && (!active || active[sb]);
+    if (!va && !vb) return;  // Cell.isActive gate (FastTYMSolver.java:51)
+    update_link_pair<I, HAS_J, REUNIT>(i, U, E, J, Unext, L, sa, sb, va, vb);
+}
+
 // The measured step: the update above plus the per-site BulkQuantities terms
 // it can form from what it loads (update_site_pair with MEAS) and the Gauss
 // law of the previous state from the previous step's transported terms Win
@@ -381,6 +413,18 @@ static void update_grid_su3f_pair_i(Ctx &c, bool reunit) {
     dim3 grid(grid_for(threads, B));
     const float *U = (const float *)c.U, *J = (const float *)c.J;
     float *E = (float *)c.E, *Un = (float *)c.Unext;
+    if (c.L.V <= LINK_WARPS_MAX_V) {
+        const dim3 g((unsigned)((3 * ((c.L.V + 63) / 64) + 3) / 4));
+        if (c.j_nonzero) {
+            if (reunit) k_update_link_su3f_pair<I, true, true><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            else k_update_link_su3f_pair<I, true, false><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        } else {
+            if (reunit) k_update_link_su3f_pair<I, false, true><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            else k_update_link_su3f_pair<I, false, false><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        }
+        c.launches++;
+        return;
+    }
     if (c.j_nonzero) {
         if (reunit) k_update_grid_su3f_pair<I, true, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
         else k_update_grid_su3f_pair<I, true, false><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);

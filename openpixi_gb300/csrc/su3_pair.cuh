@@ -606,7 +606,7 @@ template <typename I> __device__ __forceinline__ void coords(const Lat &L, I s, 
 constexpr int MEAS_THREADS = 128;
 constexpr int MEAS_COLS = 7;
 
-// FastTYMSolver.CombinedUpdate for SU(3) FP32 at sites sa and sb; a lane
+// FastTYMSolver.CombinedUpdate for SU(3) FP32, link i of sites sa and sb; a lane
 // whose flag (va, vb) is false computes but stores nothing (a site past the end
 // of the lattice or an inactive cell).  Same equations and staple order as
 // update_site in leapfrog.cuh.
@@ -621,7 +621,7 @@ constexpr int MEAS_COLS = 7;
 // stores W_i(x) = U_i(x)^dagger E_i(x) U_i(x) (its input link, the new E) in
 // Wout: the transported term that the next step reads at x + i.
 template <typename I, bool HAS_J, bool REUNIT, bool MEAS = false>
-__device__ __forceinline__ void update_site_pair(const float *__restrict__ U, float *__restrict__ E,
+__device__ __forceinline__ void update_link_pair(int i, const float *__restrict__ U, float *__restrict__ E,
                                                  const float *__restrict__ J, float *__restrict__ Unext,
                                                  const Lat &L, I sa, I sb, bool va, bool vb,
                                                  float *__restrict__ Eout = nullptr, float *slot = nullptr,
@@ -633,8 +633,7 @@ __device__ __forceinline__ void update_site_pair(const float *__restrict__ U, fl
     coords<I>(L, sb, xb);
     const Deltas<I> Da = deltas<I>(L, xa), Db = deltas<I>(L, xb);
     const P dt = bc(L.dtf), mdt = bc(-L.dtf);
-#pragma unroll 1
-    for (int i = 0; i < 3; i++) {
+    {
         const I pia = sa + Da.f(i), pib = sb + Db.f(i);  // x + i
         M S = mzero();
         [[maybe_unused]] M Pl;  // MEAS: the forward staple of plane i + 1
@@ -725,6 +724,17 @@ __device__ __forceinline__ void update_site_pair(const float *__restrict__ U, fl
         if (REUNIT) reunit(Vn);
         store<I>(Unext, nblk, i, sa, sb, va, vb, Vn);
     }
+}
+
+// The three links of the two sites
+template <typename I, bool HAS_J, bool REUNIT, bool MEAS = false>
+__device__ __forceinline__ void update_site_pair(const float *__restrict__ U, float *__restrict__ E,
+                                                 const float *__restrict__ J, float *__restrict__ Unext,
+                                                 const Lat &L, I sa, I sb, bool va, bool vb,
+                                                 float *__restrict__ Eout = nullptr, float *slot = nullptr,
+                                                 float *__restrict__ Wout = nullptr) {
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) update_link_pair<I, HAS_J, REUNIT, MEAS>(i, U, E, J, Unext, L, sa, sb, va, vb, Eout, slot, Wout);
 }
 
 // Gauss-law square of the state before a step (Grid.getGaussConstraintSquared,
