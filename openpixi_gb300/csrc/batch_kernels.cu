@@ -135,6 +135,7 @@ template <> struct FlatBounds<2, float> { static constexpr int minb = 4; };
 template <int NC, typename R, typename I, bool REUNIT>
 __global__ void __launch_bounds__(256, FlatBounds<NC, R>::minb) k_batch_flat(const BEvent<R> *__restrict__ ev, const int *__restrict__ order,
                                                     const int *__restrict__ bstart, int nev, int rd) {
+    pdl_wait();
     const int q = flat_event(bstart, nev, (int)blockIdx.x);
     const BEvent<R> &e = ev[order[q]];
     const I s = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
@@ -148,6 +149,7 @@ template <typename I, bool REUNIT>
 __global__ void __launch_bounds__(128, 3) k_batch_flat_su3f(const BEvent<float> *__restrict__ ev,
                                                             const int *__restrict__ order,
                                                             const int *__restrict__ bstart, int nev, int rd) {
+    pdl_wait();
     const int q = flat_event(bstart, nev, (int)blockIdx.x);
     const BEvent<float> &e = ev[order[q]];
     const I t = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
@@ -344,7 +346,17 @@ static cudaError_t launch_flat(Batch &b, int nsteps, cudaStream_t st) {
         void *args[] = {(void *)&ev, (void *)&order, (void *)&bstart, (void *)&nev, (void *)&rd};
         void *kf = b.int_offsets ? (reunit ? flat_kernel<NC, R, int, true>() : flat_kernel<NC, R, int, false>())
                                  : (reunit ? flat_kernel<NC, R, long, true>() : flat_kernel<NC, R, long, false>());
-        cudaError_t e = cudaLaunchKernel(kf, dim3(b.flat_blocks), dim3(b.block), args, 0, st);
+        // the steps overlap as in launch_pdl (in a captured graph too)
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(b.flat_blocks);
+        cfg.blockDim = dim3(b.block);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = b.flat_blocks >= 3 * 152 ? 1 : 0;
+        cudaError_t e = cudaLaunchKernelExC(&cfg, kf, args);
         b.launches++;
         if (e != cudaSuccess) return e;
     }

@@ -38,6 +38,7 @@ template <int NC, typename R, bool HAS_J, bool REUNIT, typename I, bool PLANES =
 __global__ void __launch_bounds__(128, UpdateBounds<NC, R>::minb)
 k_update_grid(const R *__restrict__ U, R *__restrict__ E, const R *__restrict__ J, R *__restrict__ Unext,
               const uint8_t *__restrict__ active, Lat L) {
+    pdl_wait();
     const I s = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
     if (s >= (I)L.V) return;
     if (active && !active[s]) return;  // Cell.isActive gate (FastTYMSolver.java:51)
@@ -58,6 +59,7 @@ template <typename I, bool HAS_J, bool REUNIT>
 __global__ void __launch_bounds__(128, 3)
 k_update_grid_su3f_pair(const float *__restrict__ U, float *__restrict__ E, const float *__restrict__ J,
                         float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L) {
+    pdl_wait();
     const I t = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
     const I sa = ((t >> 5) << 6) + (t & 31);
     {
@@ -94,6 +96,7 @@ template <typename I, bool HAS_J, bool REUNIT>
 __global__ void __launch_bounds__(128, 3)
 k_update_link_su3f_pair(const float *__restrict__ U, float *__restrict__ E, const float *__restrict__ J,
                         float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L) {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const unsigned w = blockIdx.x * 4u + (threadIdx.x >> 5);
     const int i = (int)(w % 3u);
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(MEAS_THREADS, 3)
 k_update_measure_su3f_pair(const float *__restrict__ U, float *__restrict__ E, float *__restrict__ Eout,
                            const float *__restrict__ Win, float *__restrict__ Wout, const float *__restrict__ rho,
                            float *__restrict__ Unext, Lat L, double *__restrict__ part) {
+    pdl_wait();
     __shared__ float slots[MEAS_COLS * MEAS_THREADS];
     float *slot = slots + threadIdx.x;
 #pragma unroll
@@ -201,11 +205,11 @@ void launch_update_measure(Ctx &c, bool reunit, void *Eout, const void *Win, voi
     const float *Wi = (const float *)Win;
     float *E = (float *)c.E, *Eo = (float *)Eout, *Un = (float *)c.Unext, *Wo = (float *)Wout;
     if (c.int_offsets) {
-        if (reunit) k_update_measure_su3f_pair<int, true><<<nb, MEAS_THREADS, 0, c.stream>>>(U, E, Eo, Wi, Wo, rho, Un, c.L, part);
-        else k_update_measure_su3f_pair<int, false><<<nb, MEAS_THREADS, 0, c.stream>>>(U, E, Eo, Wi, Wo, rho, Un, c.L, part);
+        if (reunit) launch_pdl(false, k_update_measure_su3f_pair<int, true>, nb, MEAS_THREADS, c.stream, U, E, Eo, Wi, Wo, rho, Un, c.L, part);
+        else launch_pdl(false, k_update_measure_su3f_pair<int, false>, nb, MEAS_THREADS, c.stream, U, E, Eo, Wi, Wo, rho, Un, c.L, part);
     } else {
-        if (reunit) k_update_measure_su3f_pair<long, true><<<nb, MEAS_THREADS, 0, c.stream>>>(U, E, Eo, Wi, Wo, rho, Un, c.L, part);
-        else k_update_measure_su3f_pair<long, false><<<nb, MEAS_THREADS, 0, c.stream>>>(U, E, Eo, Wi, Wo, rho, Un, c.L, part);
+        if (reunit) launch_pdl(false, k_update_measure_su3f_pair<long, true>, nb, MEAS_THREADS, c.stream, U, E, Eo, Wi, Wo, rho, Un, c.L, part);
+        else launch_pdl(false, k_update_measure_su3f_pair<long, false>, nb, MEAS_THREADS, c.stream, U, E, Eo, Wi, Wo, rho, Un, c.L, part);
     }
     c.launches += 1;
 }
@@ -360,8 +364,8 @@ static int implicit_update_t(Ctx &c) {
     // ImplicitBegin (:68-90): the explicit combined update into the implicit grid
     const int B = 128;
     const dim3 grid(grid_for(V, B));
-    if (c.j_nonzero) k_update_grid<NC, R, true, false, long><<<grid, B, 0, c.stream>>>((const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
-    else k_update_grid<NC, R, false, false, long><<<grid, B, 0, c.stream>>>((const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
+    if (c.j_nonzero) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
+    else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
     c.launches++;
     for (int it = 0; it < c.imp_iterations; it++) {
         std::swap(Ui, Uin);  // implicitGrid.storeFields()
@@ -416,21 +420,21 @@ static void update_grid_su3f_pair_i(Ctx &c, bool reunit) {
     if (c.L.V <= LINK_WARPS_MAX_V) {
         const dim3 g((unsigned)((3 * ((c.L.V + 63) / 64) + 3) / 4));
         if (c.j_nonzero) {
-            if (reunit) k_update_link_su3f_pair<I, true, true><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-            else k_update_link_su3f_pair<I, true, false><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, true, true>, g, B, c.stream, U, E, J, Un, c.active, c.L);
+            else launch_pdl(false, k_update_link_su3f_pair<I, true, false>, g, B, c.stream, U, E, J, Un, c.active, c.L);
         } else {
-            if (reunit) k_update_link_su3f_pair<I, false, true><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-            else k_update_link_su3f_pair<I, false, false><<<g, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, false, true>, g, B, c.stream, U, E, J, Un, c.active, c.L);
+            else launch_pdl(false, k_update_link_su3f_pair<I, false, false>, g, B, c.stream, U, E, J, Un, c.active, c.L);
         }
         c.launches++;
         return;
     }
     if (c.j_nonzero) {
-        if (reunit) k_update_grid_su3f_pair<I, true, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-        else k_update_grid_su3f_pair<I, true, false><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, true, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        else launch_pdl(false, k_update_grid_su3f_pair<I, true, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
     } else {
-        if (reunit) k_update_grid_su3f_pair<I, false, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-        else k_update_grid_su3f_pair<I, false, false><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, false, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        else launch_pdl(false, k_update_grid_su3f_pair<I, false, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
     }
     c.launches++;
 }
@@ -481,20 +485,20 @@ static void launch_update_grid_i(Ctx &c, bool reunit, dim3 grid, int B, const R 
     // in FP64, 5 % in FP32)
     if (NC == 2) {
         if (c.j_nonzero) {
-            if (reunit) k_update_grid<NC, R, true, true, I, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-            else k_update_grid<NC, R, true, false, I, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
         } else {
-            if (reunit) k_update_grid<NC, R, false, true, I, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-            else k_update_grid<NC, R, false, false, I, true><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
         }
         return;
     }
     if (c.j_nonzero) {
-        if (reunit) k_update_grid<NC, R, true, true, I><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-        else k_update_grid<NC, R, true, false, I><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
     } else {
-        if (reunit) k_update_grid<NC, R, false, true, I><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
-        else k_update_grid<NC, R, false, false, I><<<grid, B, 0, c.stream>>>(U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
     }
 }
 
@@ -522,8 +526,8 @@ static void update_grid_fx(Ctx &c) {
     ensure_fixed_links(c, true, false);
     const int2 *F = (const int2 *)c.fx_U;
     int2 *Fn = (int2 *)c.fx_Unext;
-    if (c.j_nonzero) fx::k_update_links_fx<NC, true, I><<<nb, B, 0, c.stream>>>(F, U, E, J, Un, Fn, c.active, c.L);
-    else fx::k_update_links_fx<NC, false, I><<<nb, B, 0, c.stream>>>(F, U, E, J, Un, Fn, c.active, c.L);
+    if (c.j_nonzero) launch_pdl(false, fx::k_update_links_fx<NC, true, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L);
+    else launch_pdl(false, fx::k_update_links_fx<NC, false, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L);
     c.fx_Unext_ok = c.active == nullptr;
     c.launches++;
 }

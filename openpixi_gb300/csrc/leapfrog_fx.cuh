@@ -22,6 +22,7 @@
 // by row at 128 (both before the multiply-adds were written in asm, 0.492).
 #pragma once
 #include "fixed.cuh"
+#include "internal.h"
 #include "leapfrog.cuh"
 
 namespace opx {
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(128, FxBounds<NC>::minb)
 k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, double *__restrict__ E,
                   const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf,
                   const uint8_t *__restrict__ active, const __grid_constant__ Lat L) {
+    pdl_wait();
     const unsigned chunk = blockIdx.x / 3u;
     const int i = (int)(blockIdx.x - 3u * chunk);
     const I s = (I)chunk * (I)blockDim.x + (I)threadIdx.x;
