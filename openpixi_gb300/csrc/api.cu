@@ -98,6 +98,23 @@ static void release(Ctx &c) {
     if (c.stream) cudaStreamDestroy(c.stream);
 }
 
+// The device address of a page-locked host buffer of n doubles (cudaMallocHost
+// or cudaHostRegister memory, both ends mapped at one offset), or null for
+// pageable memory.  The conversion kernels read and write page-locked buffers
+// directly over the host link; pageable ones go through the staging copy.
+double *opx::device_view(const void *host, size_t n) {
+    cudaPointerAttributes a0, a1;
+    const char *first = (const char *)host, *last = first + n * sizeof(double) - 1;
+    if (cudaPointerGetAttributes(&a0, first) != cudaSuccess || cudaPointerGetAttributes(&a1, last) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (a0.type != cudaMemoryTypeHost || a1.type != cudaMemoryTypeHost || !a0.devicePointer || !a1.devicePointer)
+        return nullptr;
+    if ((const char *)a1.devicePointer - (const char *)a0.devicePointer != last - first) return nullptr;
+    return (double *)a0.devicePointer;
+}
+
 extern "C" {
 
 int opx_version(void) { return 10000; }
@@ -222,23 +239,6 @@ static int field_count(const Ctx &c, int field, int layout, size_t *n, int *ndir
     case OPX_FIELD_RHO: *n = (size_t)c.L.V * na_host; *ndir = 1; return OPX_OK;
     }
     return OPX_ERR_INVALID;
-}
-
-// The device address of a page-locked host buffer of n doubles (cudaMallocHost
-// or cudaHostRegister memory, both ends mapped at one offset), or null for
-// pageable memory.  The conversion kernels read and write page-locked buffers
-// directly over the host link; pageable ones go through the staging copy.
-static double *device_view(const void *host, size_t n) {
-    cudaPointerAttributes a0, a1;
-    const char *first = (const char *)host, *last = first + n * sizeof(double) - 1;
-    if (cudaPointerGetAttributes(&a0, first) != cudaSuccess || cudaPointerGetAttributes(&a1, last) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a0.type != cudaMemoryTypeHost || a1.type != cudaMemoryTypeHost || !a0.devicePointer || !a1.devicePointer)
-        return nullptr;
-    if ((const char *)a1.devicePointer - (const char *)a0.devicePointer != last - first) return nullptr;
-    return (double *)a0.devicePointer;
 }
 
 int opx_upload(opx_ctx *ctx, int field, const double *host, size_t count, int layout) {

@@ -211,6 +211,8 @@ void launch_energy_density(Ctx &c, double *dev_out);
 void launch_projected_energy(Ctx &c, int dir, int skip_u, const double *bn_site, double *dev_out);
 int launch_projected_poynting(Ctx &c, int dir, double *dev_out);  // SU(2) only
 void launch_gauss_field(Ctx &c, double *dev_out);
+// The device address of a page-locked host buffer of n doubles, or null (api.cu)
+double *device_view(const void *host, size_t n);
 // ---- conversions (convert_kernels.cu) ----
 void launch_links_from_ref(Ctx &c, const double *src, void *dst);
 void launch_links_to_ref(Ctx &c, const void *src, double *dst);
