@@ -623,8 +623,8 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
     };
     auto step64 = [&](const int2 *F, const double *W, double *E, double *Wn, int2 *Fn) {
         if (!fixed) k_step_plain<2, double, false><<<gs, 128, 0, c.stream>>>(W, E, Wn, c.L);
-        else if (c.int_offsets) launch_pdl(false, fx::k_update_links_fx<2, false, int>, 3 * gs.x, 128, c.stream, F, W, E, nullptr, Wn, Fn, nullptr, c.L);
-        else launch_pdl(false, fx::k_update_links_fx<2, false, long>, 3 * gs.x, 128, c.stream, F, W, E, nullptr, Wn, Fn, nullptr, c.L);
+        else if (c.int_offsets) launch_pdl(false, fx::k_update_links_fx<2, false, int>, 3 * gs.x, 128, c.stream, F, W, E, nullptr, Wn, Fn, nullptr, c.L, nullptr);
+        else launch_pdl(false, fx::k_update_links_fx<2, false, long>, 3 * gs.x, 128, c.stream, F, W, E, nullptr, Wn, Fn, nullptr, c.L, nullptr);
         c.launches++;
     };
     auto store_ckpt = [&](int k, char *W) {

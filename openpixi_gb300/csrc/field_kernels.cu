@@ -37,8 +37,9 @@ template <> struct UpdateBounds<2, float> { static constexpr int minb = 8; };
 template <int NC, typename R, bool HAS_J, bool REUNIT, typename I, bool PLANES = false>
 __global__ void __launch_bounds__(128, UpdateBounds<NC, R>::minb)
 k_update_grid(const R *__restrict__ U, R *__restrict__ E, const R *__restrict__ J, R *__restrict__ Unext,
-              const uint8_t *__restrict__ active, Lat L) {
+              const uint8_t *__restrict__ active, Lat L, const unsigned *stop) {
     pdl_wait();
+    if (stopped(stop)) return;
     const I s = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
     if (s >= (I)L.V) return;
     if (active && !active[s]) return;  // Cell.isActive gate (FastTYMSolver.java:51)
@@ -58,8 +59,9 @@ k_update_grid(const R *__restrict__ U, R *__restrict__ E, const R *__restrict__ 
 template <typename I, bool HAS_J, bool REUNIT>
 __global__ void __launch_bounds__(128, 3)
 k_update_grid_su3f_pair(const float *__restrict__ U, float *__restrict__ E, const float *__restrict__ J,
-                        float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L) {
+                        float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L, const unsigned *stop) {
     pdl_wait();
+    if (stopped(stop)) return;
     const I t = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
     const I sa = ((t >> 5) << 6) + (t & 31);
     {
@@ -95,8 +97,9 @@ constexpr long LINK_WARPS_MAX_V = 1000000;
 template <typename I, bool HAS_J, bool REUNIT>
 __global__ void __launch_bounds__(128, 3)
 k_update_link_su3f_pair(const float *__restrict__ U, float *__restrict__ E, const float *__restrict__ J,
-                        float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L) {
+                        float *__restrict__ Unext, const uint8_t *__restrict__ active, Lat L, const unsigned *stop) {
     pdl_wait();
+    if (stopped(stop)) return;
     const int lane = threadIdx.x & 31;
     const unsigned w = blockIdx.x * 4u + (threadIdx.x >> 5);
     const int i = (int)(w % 3u);
@@ -364,8 +367,8 @@ static int implicit_update_t(Ctx &c) {
     // ImplicitBegin (:68-90): the explicit combined update into the implicit grid
     const int B = 128;
     const dim3 grid(grid_for(V, B));
-    if (c.j_nonzero) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
-    else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L);
+    if (c.j_nonzero) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L, (const unsigned *)nullptr);
+    else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, long>, grid, B, c.stream, (const R *)c.U, Ei, (const R *)c.J, Uin, c.active, c.L, (const unsigned *)nullptr);
     c.launches++;
     for (int it = 0; it < c.imp_iterations; it++) {
         std::swap(Ui, Uin);  // implicitGrid.storeFields()
@@ -420,21 +423,21 @@ static void update_grid_su3f_pair_i(Ctx &c, bool reunit) {
     if (c.L.V <= LINK_WARPS_MAX_V) {
         const dim3 g((unsigned)((3 * ((c.L.V + 63) / 64) + 3) / 4));
         if (c.j_nonzero) {
-            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, true, true>, g, B, c.stream, U, E, J, Un, c.active, c.L);
-            else launch_pdl(false, k_update_link_su3f_pair<I, true, false>, g, B, c.stream, U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, true, true>, g, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+            else launch_pdl(false, k_update_link_su3f_pair<I, true, false>, g, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
         } else {
-            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, false, true>, g, B, c.stream, U, E, J, Un, c.active, c.L);
-            else launch_pdl(false, k_update_link_su3f_pair<I, false, false>, g, B, c.stream, U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(false, k_update_link_su3f_pair<I, false, true>, g, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+            else launch_pdl(false, k_update_link_su3f_pair<I, false, false>, g, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
         }
         c.launches++;
         return;
     }
     if (c.j_nonzero) {
-        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, true, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-        else launch_pdl(false, k_update_grid_su3f_pair<I, true, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, true, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+        else launch_pdl(false, k_update_grid_su3f_pair<I, true, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
     } else {
-        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, false, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-        else launch_pdl(false, k_update_grid_su3f_pair<I, false, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(false, k_update_grid_su3f_pair<I, false, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+        else launch_pdl(false, k_update_grid_su3f_pair<I, false, false>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
     }
     c.launches++;
 }
@@ -485,20 +488,20 @@ static void launch_update_grid_i(Ctx &c, bool reunit, dim3 grid, int B, const R 
     // in FP64, 5 % in FP32)
     if (NC == 2) {
         if (c.j_nonzero) {
-            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
         } else {
-            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+            if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+            else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I, true>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
         }
         return;
     }
     if (c.j_nonzero) {
-        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, true, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
     } else {
-        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
-        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L);
+        if (reunit) launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, true, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
+        else launch_pdl(NC == 2 && sizeof(R) == 4, k_update_grid<NC, R, false, false, I>, grid, B, c.stream, U, E, J, Un, c.active, c.L, c.status);
     }
 }
 
@@ -526,8 +529,8 @@ static void update_grid_fx(Ctx &c) {
     ensure_fixed_links(c, true, false);
     const int2 *F = (const int2 *)c.fx_U;
     int2 *Fn = (int2 *)c.fx_Unext;
-    if (c.j_nonzero) launch_pdl(false, fx::k_update_links_fx<NC, true, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L);
-    else launch_pdl(false, fx::k_update_links_fx<NC, false, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L);
+    if (c.j_nonzero) launch_pdl(false, fx::k_update_links_fx<NC, true, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L, c.status);
+    else launch_pdl(false, fx::k_update_links_fx<NC, false, I>, nb, B, c.stream, F, U, E, J, Un, Fn, c.active, c.L, c.status);
     c.fx_Unext_ok = c.active == nullptr;
     c.launches++;
 }

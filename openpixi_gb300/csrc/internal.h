@@ -42,14 +42,11 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Whether the handle's status word stops the steps queued behind a reduction that
+// found non-finite values (opx_step_measured); null: never
+__device__ __forceinline__ bool stopped(const unsigned *stop) { return stop && *(const volatile unsigned *)stop != 0u; }
 #endif
 
-// Device status word bits (read back by the host after each API call that
-// checks numerics).
-enum : unsigned {
-    STATUS_NAN = 1u,        // a NaN/Inf was produced
-    STATUS_CG_DIVERGED = 2u,
-};
 
 struct Particles {
     long n = 0, cap = 0;
@@ -124,8 +121,7 @@ struct Ctx {
     double *red_out = nullptr;     // device
     unsigned *red_count = nullptr; // device: blocks of the running reduction that have finished
     double *red_host = nullptr;    // pinned
-    unsigned *status = nullptr;    // device status word
-    unsigned *status_host = nullptr;
+    unsigned *status = nullptr;    // device: nonzero stops the steps of opx_step_measured that are queued (zero between calls)
     long steps = 0;
     long launches = 0;
     // Reuse of B^2 across reductions: a reduction after one opx_step(ctx, 1)
@@ -174,7 +170,8 @@ struct Ctx {
         const void *unext = nullptr;
     } bnsite;
     double *meas_part = nullptr, *meas_rows = nullptr, *meas_host = nullptr;  // rows: device and pinned
-    int meas_rows_cap = 0, meas_chunk = 0;  // steps whose partials meas_part holds
+    long meas_rows_cap = 0;  // doubles
+    int meas_chunk = 0;  // steps whose partials meas_part holds
     bool profiling = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double phase_ms[OPX_NUM_PHASES] = {0, 0, 0, 0};
@@ -199,9 +196,10 @@ int measured_parts(const Ctx &c);
 void launch_update_measure(Ctx &c, bool reunit, void *Eout, const void *Win, void *Wout, double *part);
 void launch_measure_combine(Ctx &c, const double *part, int nsteps, double *rows);  // rows[nsteps][8]
 // ---- reductions (reduce_kernels.cu) ----
-// result in c.red_out[0..10]: E^2[3], B^2 of U [3] (zero with skip_u), G^2, rho^2, B^2 of Unext [3]
+// columns 0..10: E^2[3], B^2 of U [3] (zero with skip_u), G^2, rho^2, B^2 of Unext [3]
 constexpr int BULK_COLUMNS = 11;
-void launch_bulk(Ctx &c, int skip_u);
+// result in out (null: c.red_out); stop: the word that non-finite sums set, or null
+void launch_bulk(Ctx &c, int skip_u, double *out = nullptr, unsigned *stop = nullptr);
 int reduction_blocks(long V);
 int bulk_blocks_max(long V);
 void launch_energy_density(Ctx &c, double *dev_out);

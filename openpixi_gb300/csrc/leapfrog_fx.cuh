@@ -273,8 +273,9 @@ template <int NC, bool HAS_J, typename I>
 __global__ void __launch_bounds__(128, FxBounds<NC>::minb)
 k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, double *__restrict__ E,
                   const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf,
-                  const uint8_t *__restrict__ active, const __grid_constant__ Lat L) {
+                  const uint8_t *__restrict__ active, const __grid_constant__ Lat L, const unsigned *stop) {
     pdl_wait();
+    if (stopped(stop)) return;
     const unsigned chunk = blockIdx.x / 3u;
     const int i = (int)(blockIdx.x - 3u * chunk);
     const I s = (I)chunk * (I)blockDim.x + (I)threadIdx.x;

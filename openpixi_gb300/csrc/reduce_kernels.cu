@@ -44,7 +44,7 @@ constexpr int NQS = BULK_COLUMNS;
 // resets the counter for the next launch on the stream.  No block waits on
 // another.
 template <int NQ>
-__device__ __forceinline__ void last_block_combine(const double *part, unsigned *count, double *out) {
+__device__ __forceinline__ void last_block_combine(const double *part, unsigned *count, double *out, unsigned *stop) {
     __shared__ bool last;
     __threadfence();
     __syncthreads();
@@ -55,7 +55,10 @@ __device__ __forceinline__ void last_block_combine(const double *part, unsigned 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
     for (int q = warp; q < NQ; q += nw) {
         const double v = warp_sum_pairs(part + 2 * q, (int)gridDim.x, 2L * NQ);
-        if (lane == 0) out[q] = v;
+        if (lane == 0) {
+            out[q] = v;
+            if (stop && !isfinite(v)) atomicOr(stop, 1u);
+        }
     }
     if (threadIdx.x == 0) *count = 0u;
 }
@@ -65,7 +68,8 @@ __global__ void __launch_bounds__(RED_THREADS, RedBounds<NC, R>::minb)
     k_bulk_partial(const R *__restrict__ U, const R *__restrict__ Unext, const R *__restrict__ E,
                    const R *__restrict__ rho, const uint8_t *__restrict__ eval, Lat L, int skip_u,
                    double *__restrict__ part, unsigned *__restrict__ count, double *__restrict__ out,
-                   double *__restrict__ bn_site) {
+                   unsigned *__restrict__ stop, double *__restrict__ bn_site) {
+    pdl_wait();
     using G = typename GroupOf<NC, R>::T;
     constexpr int NA = G::NA;
     const LinkPlanes<G, R> Up{const_cast<R *>(U), L.V}, Unp{const_cast<R *>(Unext), L.V};
@@ -132,7 +136,7 @@ __global__ void __launch_bounds__(RED_THREADS, RedBounds<NC, R>::minb)
         part[((long)blockIdx.x * NQS + q) * 2] = v.s;
         part[((long)blockIdx.x * NQS + q) * 2 + 1] = v.c;
     }
-    last_block_combine<NQS>(part, count, out);
+    last_block_combine<NQS>(part, count, out, stop);
 }
 
 // FP64 with the group products in fixed point.  Three warps share 32 sites, warp d
@@ -153,7 +157,8 @@ __global__ void __launch_bounds__(BulkFx<NC>::groups * 96, BulkFx<NC>::minb)
                       const double *__restrict__ Unext, const double *__restrict__ E, const double *__restrict__ rho,
                       const uint8_t *__restrict__ eval, const __grid_constant__ Lat L, int skip_u,
                       double *__restrict__ part, unsigned *__restrict__ count, double *__restrict__ out,
-                      double *__restrict__ bn_site) {
+                      unsigned *__restrict__ stop, double *__restrict__ bn_site) {
+    pdl_wait();
     constexpr int NA = NC == 2 ? 3 : 8, G = BulkFx<NC>::groups;
     __shared__ double sh[5][3 * G];
     __shared__ double gt[2][G][3][NA][32];
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(BulkFx<NC>::groups * 96, BulkFx<NC>::minb)
             part[((long)blockIdx.x * NQS + q) * 2 + 1] = 0.0;
         }
     }
-    last_block_combine<NQS>(part, count, out);
+    last_block_combine<NQS>(part, count, out, stop);
 }
 
 // blocks whose partials the handle's buffer holds: 32 sites each at least, 1216 at most
@@ -250,7 +255,8 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
     k_bulk_partial_su3f_pair(const float *__restrict__ U, const float *__restrict__ Unext,
                              const float *__restrict__ E, const float *__restrict__ rho,
                              const uint8_t *__restrict__ eval, Lat L, int skip_u, double *__restrict__ part,
-                             unsigned *__restrict__ count, double *__restrict__ out) {
+                             unsigned *__restrict__ count, double *__restrict__ out, unsigned *__restrict__ stop) {
+    pdl_wait();
     using namespace pr;
     const I V = (I)L.V, nblk = (I)((L.V + 31) >> 5);
     const I npairs = (I)(((L.V + 63) >> 6) << 5);
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
         part[((long)blockIdx.x * NQS + q) * 2] = v.s;
         part[((long)blockIdx.x * NQS + q) * 2 + 1] = v.c;
     }
-    last_block_combine<NQS>(part, count, out);
+    last_block_combine<NQS>(part, count, out, stop);
 }
 
 
@@ -398,23 +404,22 @@ static int resident_blocks(K kernel, int threads = RED_THREADS) {
 }
 
 template <int NC, typename I>
-static void bulk_fx(Ctx &c, int skip_u) {
+static void bulk_fx(Ctx &c, int skip_u, double *out, unsigned *stop) {
     constexpr int T = BulkFx<NC>::groups * 96;
     static const int wave = resident_blocks(k_bulk_partial_fx<NC, I>, T);
     const long want = (c.L.V + BulkFx<NC>::groups * 32 - 1) / (BulkFx<NC>::groups * 32);
     const int nb = (int)std::min<long>(std::min(bulk_blocks_max(c.L.V), wave), want);
     ensure_fixed_links(c, true, true);
-    k_bulk_partial_fx<NC, I><<<nb, T, 0, c.stream>>>(
-        (const int2 *)c.fx_U, (const int2 *)c.fx_Unext, (const double *)c.U, (const double *)c.Unext, (const double *)c.E,
-        (const double *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L, skip_u, c.red_part, c.red_count, c.red_out, c.bn_site);
+    launch_pdl(false, k_bulk_partial_fx<NC, I>, nb, T, c.stream, (const int2 *)c.fx_U, (const int2 *)c.fx_Unext, (const double *)c.U, (const double *)c.Unext, (const double *)c.E,
+        (const double *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L, skip_u, c.red_part, c.red_count, out, stop, c.bn_site);
     c.launches += 1;
 }
 
 template <int NC, typename R>
-static void bulk_t(Ctx &c, int skip_u) {
+static void bulk_t(Ctx &c, int skip_u, double *out, unsigned *stop) {
     if (sizeof(R) == 8 && c.fixed_kernel) {
-        if (c.int_offsets) bulk_fx<NC, int>(c, skip_u);
-        else bulk_fx<NC, long>(c, skip_u);
+        if (c.int_offsets) bulk_fx<NC, int>(c, skip_u, out, stop);
+        else bulk_fx<NC, long>(c, skip_u, out, stop);
         return;
     }
     int nb = c.red_blocks;
@@ -422,31 +427,30 @@ static void bulk_t(Ctx &c, int skip_u) {
         if (c.int_offsets) {
             static const int wave = resident_blocks(k_bulk_partial_su3f_pair<int>);
             nb = std::min(nb, wave);
-            k_bulk_partial_su3f_pair<int><<<nb, RED_THREADS, 0, c.stream>>>(
-                (const float *)c.U, (const float *)c.Unext, (const float *)c.E, (const float *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L,
-                skip_u, c.red_part, c.red_count, c.red_out);
+            launch_pdl(false, k_bulk_partial_su3f_pair<int>, nb, RED_THREADS, c.stream, (const float *)c.U, (const float *)c.Unext, (const float *)c.E, (const float *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L,
+                skip_u, c.red_part, c.red_count, out, stop);
         } else {
             static const int wave = resident_blocks(k_bulk_partial_su3f_pair<long>);
             nb = std::min(nb, wave);
-            k_bulk_partial_su3f_pair<long><<<nb, RED_THREADS, 0, c.stream>>>(
-                (const float *)c.U, (const float *)c.Unext, (const float *)c.E, (const float *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L,
-                skip_u, c.red_part, c.red_count, c.red_out);
+            launch_pdl(false, k_bulk_partial_su3f_pair<long>, nb, RED_THREADS, c.stream, (const float *)c.U, (const float *)c.Unext, (const float *)c.E, (const float *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L,
+                skip_u, c.red_part, c.red_count, out, stop);
         }
     } else {
         static const int wave = resident_blocks(k_bulk_partial<NC, R>);
         nb = std::min(nb, wave);
-        k_bulk_partial<NC, R><<<nb, RED_THREADS, 0, c.stream>>>((const R *)c.U, (const R *)c.Unext, (const R *)c.E,
+        launch_pdl(false, k_bulk_partial<NC, R>, nb, RED_THREADS, c.stream, (const R *)c.U, (const R *)c.Unext, (const R *)c.E,
                                                                (const R *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L, skip_u, c.red_part,
-                                                               c.red_count, c.red_out, c.bn_site);
+                                                               c.red_count, out, stop, c.bn_site);
     }
     c.launches += 1;
 }
 
-void launch_bulk(Ctx &c, int skip_u) {
+void launch_bulk(Ctx &c, int skip_u, double *out, unsigned *stop) {
+    if (!out) out = c.red_out;
     if (c.nc == 2) {
-        if (c.prec == OPX_F64) bulk_t<2, double>(c, skip_u); else bulk_t<2, float>(c, skip_u);
+        if (c.prec == OPX_F64) bulk_t<2, double>(c, skip_u, out, stop); else bulk_t<2, float>(c, skip_u, out, stop);
     } else {
-        if (c.prec == OPX_F64) bulk_t<3, double>(c, skip_u); else bulk_t<3, float>(c, skip_u);
+        if (c.prec == OPX_F64) bulk_t<3, double>(c, skip_u, out, stop); else bulk_t<3, float>(c, skip_u, out, stop);
     }
 }
 
