@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256, FlatBounds<NC, R>::minb) k_batch_flat(con
     const BEvent<R> &e = ev[order[q]];
     const I s = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
     if (s >= (I)e.L.V) return;
-    if constexpr (NC == 2) update_site_su2_planes<R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s);
+    if constexpr (NC == 2) update_site_su2_planes<R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s, (long)nev * e.L.V >= 500000);
     else update_site<NC, R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s);
 }
 
@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(128, 3) k_batch_flat_su3f(const BEvent<float> 
     const BEvent<float> &e = ev[order[q]];
     const I t = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
     const I V = (I)e.L.V, sa = ((t >> 5) << 6) + (t & 31);
+    if ((long)nev * e.L.V >= 200000) prefetch_e_pair<I>(e.E, e.L, sa);  // 312 B a site: the batch is not held in L2
     if (sa >= V) return;
     I sb = sa + 32;
     const bool vb = sb < V;

@@ -30,8 +30,9 @@ int grid_for(long n, int block) { return (int)((n + block - 1) / block); }
 template <int NC, typename R> struct UpdateBounds { static constexpr int minb = 4; };
 template <> struct UpdateBounds<3, double> { static constexpr int minb = 3; };
 // SU(2) FP32 is latency-bound on its link loads: the plane-by-plane staple sums
-// at 8 blocks per SM (64 registers) take a 128^3 step in 0.081 ms (0.085 ms
-// for the per-link sums at 12 blocks and 40 registers, 0.092 ms at 56)
+// at 8 blocks per SM (64 registers) and the E prefetch take a 128^3 step in 0.071
+// ms (0.080 ms without the prefetch; without it the per-link sums at 12 blocks and
+// 40 registers 0.085 ms, at 56 0.092 ms)
 template <> struct UpdateBounds<2, float> { static constexpr int minb = 8; };
 
 template <int NC, typename R, bool HAS_J, bool REUNIT, typename I, bool PLANES = false>
@@ -45,7 +46,8 @@ k_update_grid(const R *__restrict__ U, R *__restrict__ E, const R *__restrict__ 
     if (active && !active[s]) return;  // Cell.isActive gate (FastTYMSolver.java:51)
     if constexpr (NC == 2) {
         if (PLANES) {
-            update_site_su2_planes<R, HAS_J, REUNIT, I>(U, E, J, Unext, L, s);
+            // 132 B a site: half a million sites fill half of L2 (64^3, in L2: 2 % slower with the prefetch)
+            update_site_su2_planes<R, HAS_J, REUNIT, I>(U, E, J, Unext, L, s, L.V >= 500000);
             return;
         }
     }
@@ -64,19 +66,7 @@ k_update_grid_su3f_pair(const float *__restrict__ U, float *__restrict__ E, cons
     if (stopped(stop)) return;
     const I t = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
     const I sa = ((t >> 5) << 6) + (t & 31);
-    {
-        // L2 prefetch of the warp's E lines (3 links x 8 components x the two
-        // 32-site halves), which the thread reads only after its staple sums:
-        // their DRAM latency then overlaps the staples (0.5 % per 128^3 step)
-        const int lane = threadIdx.x & 31;
-        const I s0 = sa - (I)lane + (I)((lane & 1) << 5);
-        if (lane < 16 && s0 < (I)L.V) {
-            const float *e = E + (I)(lane >> 1) * (I)L.V + s0;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(e));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(e + (I)8 * (I)L.V));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(e + (I)16 * (I)L.V));
-        }
-    }
+    prefetch_e_pair<I>(E, L, sa);
     if (sa >= (I)L.V) return;
     I sb = sa + 32;
     bool vb = sb < (I)L.V;

@@ -85,9 +85,17 @@ __device__ __forceinline__ void update_site(const R *__restrict__ U, R *__restri
 template <typename R, bool HAS_J, bool REUNIT, typename I = long>
 __device__ __forceinline__ void update_site_su2_planes(const R *__restrict__ U, R *__restrict__ E,
                                                        const R *__restrict__ J, R *__restrict__ Unext, const Lat &L,
-                                                       I s) {
+                                                       I s, bool cold = false) {
     using G = SU2<R>;
     using M = typename G::M;
+    if constexpr (sizeof(R) == 4) {
+        // cold (the fields do not stay in L2): the warp's nine E lines come to L2 while
+        // the staples are formed; read only after them, they were a second DRAM
+        // latency that 32 warps per SM did not cover (128^3 0.0796 -> 0.0708 ms a step,
+        // 256^3 0.603 -> 0.536; the links' own lines too, or to L1: no further gain)
+        const int lane = threadIdx.x & 31;
+        if (cold && lane < 9) asm volatile("prefetch.global.L2 [%0];" ::"l"(E + ((I)lane * (I)L.V + s - lane)));
+    }
     int x[3];
     site_coords<I>(L, s, x);
     const Deltas<I> D = deltas<I>(L, x);
