@@ -6,9 +6,10 @@
 //       One pass computes all of them (the reference makes six lattice passes).
 //       Per-site values are formed in the storage precision; each thread
 //       accumulates them in FP64 with compensated (Neumaier/TwoSum) sums (FP64
-//       storage) or in FP32 Kahan runs added to an FP64 sum (FP32 storage); a
+//       storage) or in FP32 pairs in runs added to an FP64 sum (FP32 storage); a
 //       block adds its threads in a fixed FP64 tree and the block partials are
 //       combined by one block in a fixed order, so results are deterministic.
+//   k_bulk_partial_su2f : the same for SU(2) FP32
 //   k_bulk_partial_fx  : the same for FP64 storage with the group products in
 //       fixed point (fixed.cuh), four threads a site
 //   k_energy_density   : EnergyDensity.ComponentComputation (EnergyDensity.java:119-166)
@@ -239,6 +240,157 @@ __global__ void __launch_bounds__(BulkFx<NC>::groups * 96, BulkFx<NC>::minb)
     last_block_combine<NQS>(part, count, out, stop);
 }
 
+// SU(2) FP32: one site per thread, the three planes and both times unrolled so that
+// they share their links (9 loads a time instead of 12) and all loads are in flight
+// together, 32-bit offsets where they fit.  A reduction moves 132 B a site and is
+// bound by its link loads like the leapfrog; the generic kernel's FP64 conversion
+// and addition per column and site and its rolled loop took 0.221 ms at 128^3 after
+// a step against 0.117 (64^3 0.085 / 0.061, 192^3 0.595 / 0.296, the host's wait
+// included).  Per-site values are FP32; a thread adds runs of 32 of
+// them as exact FP32 pairs (TwoSum, the errors summed apart), a warp its lanes'
+// runs by warp_sum and lane 0 these with compensation.  Values that could take a
+// run out of FP32's range (and what is not finite) go to the FP64 sums directly.
+template <typename I>
+__global__ void __launch_bounds__(RED_THREADS, 4)
+    k_bulk_partial_su2f(const float *__restrict__ U, const float *__restrict__ Unext, const float *__restrict__ E,
+                        const float *__restrict__ rho, const uint8_t *__restrict__ eval, const __grid_constant__ Lat L,
+                        int skip_u, double *__restrict__ part, unsigned *__restrict__ count, double *__restrict__ out,
+                        unsigned *__restrict__ stop, double *__restrict__ bn_site) {
+    pdl_wait();
+    using G = SU2<float>;
+    using M = G::M;
+    constexpr int NW = RED_THREADS / 32;
+    __shared__ KSum sums[NQS][NW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane < NQS) sums[lane][warp] = KSum{0.0, 0.0};
+    __syncwarp();
+    const I V = (I)L.V, ngroups = (I)((L.V + 31) >> 5);
+    const LinkPlanes<G, float, I> Up{const_cast<float *>(U), V};
+    const AlgPlanes<3, float, I> Ep{const_cast<float *>(E), V};
+    float hi[NQS], lo[NQS];
+#pragma unroll
+    for (int q = 0; q < NQS; q++) { hi[q] = 0.f; lo[q] = 0.f; }
+    auto to_sums = [&](int q, double x) {
+        const double v = warp_sum(x);
+        if (lane == 0) two_sum_add(sums[q][warp], v);
+    };
+    auto flush = [&]() {
+#pragma unroll
+        for (int q = 0; q < NQS; q++) {
+            to_sums(q, (double)hi[q] + (double)lo[q]);
+            hi[q] = 0.f;
+            lo[q] = 0.f;
+        }
+    };
+    int run = 0;
+    for (I g = (I)blockIdx.x * NW + warp; g < ngroups; g += (I)gridDim.x * NW) {
+        // L2 prefetch of the lines of the warp's next 32 sites: 16 warps per SM do not
+        // cover the DRAM latency (E's alone: 128^3 measured step 0.184 -> 0.182 ms, with
+        // Unext's 0.178, with both times' 0.173)
+        const I gn = g + (I)gridDim.x * NW;
+        if ((gn + 1) * 32 <= V) {
+            if (lane < 9) asm volatile("prefetch.global.L2 [%0];" ::"l"(E + ((I)lane * V + gn * 32)));
+            if (lane < 12) {
+                const I o = ((I)(lane >> 2) * V + gn * 32 + (lane & 3) * 8) * 4;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(Unext + o));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(U + o));
+            }
+        }
+        const I s = g * 32 + lane;
+        float v[NQS];
+#pragma unroll
+        for (int q = 0; q < NQS; q++) v[q] = 0.f;
+        if (s < V && (!eval || eval[s])) {
+            int x[3];
+            site_coords<I>(L, s, x);
+            const Deltas<I> D = deltas<I>(L, x);
+#pragma unroll 1
+            for (int tt = skip_u ? 1 : 0; tt < 2; tt++) {
+                const LinkPlanes<G, float, I> W{const_cast<float *>(tt ? Unext : U), V};
+                const M own[3] = {W.load(0, s), W.load(1, s), W.load(2, s)};
+                float b2[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    // U_j(x) U_k(x+j) U_j(x+k)^dagger U_k(x)^dagger (field_b)
+                    const int j = (d + 1) % 3, k = (d + 2) % 3;
+                    const M P = G::mul_adj(G::mul_adj(G::mul(own[j], W.load(k, s + D.f(j))), W.load(j, s + D.f(k))), own[k]);
+                    float b[3];
+                    G::proj(P, b);
+                    const float f = LatR<float>::bfac(L, d);
+#pragma unroll
+                    for (int a = 0; a < 3; a++) b[a] *= f;
+                    b2[d] = (float)sqr<float, 3>(b);
+                }
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    if (tt == 0) {
+                        v[3 + d] = b2[d];
+                    } else {
+                        v[8 + d] = b2[d];
+                        if (bn_site) bn_site[(long)d * L.V + s] = (double)b2[d];
+                    }
+                }
+            }
+            float gs[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const I sm = s + D.b(i);
+                float e0[3], e1[3], t[3];
+                Ep.load_ro(i, s, e0);
+                Ep.load_ro(i, sm, e1);
+                v[i] = (float)sqr<float, 3>(e0);
+                G::act(e1, G::adj(Up.load(i, sm)), t);
+                const float f = LatR<float>::gfac(L, i);
+#pragma unroll
+                for (int a = 0; a < 3; a++) gs[a] += (e0[a] - t[a]) * f;
+            }
+            if (rho) {
+                float r[3];
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    r[a] = __ldg(rho + (I)a * V + s);
+                    gs[a] -= r[a];
+                }
+                v[7] = (float)sqr<float, 3>(r);
+            }
+            v[6] = (float)sqr<float, 3>(gs);
+        }
+        float all = v[0];
+#pragma unroll
+        for (int q = 1; q < NQS; q++) all += v[q];
+        if (__any_sync(0xffffffffu, !(all < 1e30f))) {
+#pragma unroll 1
+            for (int q = 0; q < NQS; q++) {
+                float y = v[0];
+#pragma unroll
+                for (int k = 1; k < NQS; k++) y = q == k ? v[k] : y;
+                to_sums(q, (double)y);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < NQS; q++) {
+                const float t = hi[q] + v[q], z = t - hi[q];
+                lo[q] += (hi[q] - (t - z)) + (v[q] - z);
+                hi[q] = t;
+            }
+        }
+        if ((++run & 31) == 0) flush();
+    }
+    flush();
+    __syncthreads();
+    if (threadIdx.x < NQS) {
+        const int q = threadIdx.x, i = q < 6 ? q % 3 : q - 8;
+        KSum r = sums[q][0];
+#pragma unroll
+        for (int w = 1; w < NW; w++) ksum_merge(r, sums[q][w]);
+        double f = 1.0;
+        if (q != 6 && q != 7) f = (q < 3 ? 1.0 : 0.5) * (i == 0 ? L.ufac[0] : (i == 1 ? L.ufac[1] : L.ufac[2]));
+        part[((long)blockIdx.x * NQS + q) * 2] = r.s * f;
+        part[((long)blockIdx.x * NQS + q) * 2 + 1] = r.c * f;
+    }
+    last_block_combine<NQS>(part, count, out, stop);
+}
+
 // blocks whose partials the handle's buffer holds: 32 sites each at least, 1216 at most
 int bulk_blocks_max(long V) { return (int)std::min<long>(grid_for(V, 32), 8L * 152); }
 int reduction_blocks(long V) { return (int)std::min<long>(grid_for(V, RED_THREADS), 8L * 152); }
@@ -415,8 +567,22 @@ static void bulk_fx(Ctx &c, int skip_u, double *out, unsigned *stop) {
     c.launches += 1;
 }
 
+template <typename I>
+static void bulk_su2f(Ctx &c, int skip_u, double *out, unsigned *stop) {
+    static const int wave = resident_blocks(k_bulk_partial_su2f<I>);
+    launch_pdl(false, k_bulk_partial_su2f<I>, std::min(c.red_blocks, wave), RED_THREADS, c.stream, (const float *)c.U,
+        (const float *)c.Unext, (const float *)c.E, (const float *)(c.rho_nonzero ? c.rho : nullptr), c.eval, c.L, skip_u,
+        c.red_part, c.red_count, out, stop, c.bn_site);
+    c.launches += 1;
+}
+
 template <int NC, typename R>
 static void bulk_t(Ctx &c, int skip_u, double *out, unsigned *stop) {
+    if constexpr (NC == 2 && sizeof(R) == 4) {
+        if (c.int_offsets) bulk_su2f<int>(c, skip_u, out, stop);
+        else bulk_su2f<long>(c, skip_u, out, stop);
+        return;
+    }
     if (sizeof(R) == 8 && c.fixed_kernel) {
         if (c.int_offsets) bulk_fx<NC, int>(c, skip_u, out, stop);
         else bulk_fx<NC, long>(c, skip_u, out, stop);

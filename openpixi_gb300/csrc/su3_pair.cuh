@@ -730,7 +730,7 @@ __device__ __forceinline__ void update_link_pair(int i, const float *__restrict_
 // L2 prefetch of the warp's E lines (3 links x 8 components x the two 32-site
 // halves from sa of lane 0), which the thread reads only after its staple sums:
 // their DRAM latency then overlaps the staples (0.5 % per 128^3 step, 2 % per step
-// of a batch of 1024 events of 24^3)
+// of a batch of 32 events)
 template <typename I>
 __device__ __forceinline__ void prefetch_e_pair(const float *E, const Lat &L, I sa) {
     const int lane = threadIdx.x & 31;
