@@ -238,35 +238,6 @@ struct M {
     Fx r[9], i[9];
 };
 
-// (A B)_{rq}: real or imaginary part, A = a or a^dagger, B likewise
-template <bool CA, bool CB> OPX_HD OPX_INLINE void mre(Acc &s, const M &a, const M &b, int r, int q) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int x = CA ? 3 * k + r : 3 * r + k, y = CB ? 3 * q + k : 3 * k + q;
-        mac(s, a.r[x], b.r[y]);
-        mac(s, CA == CB ? neg(a.i[x]) : a.i[x], b.i[y]);
-    }
-}
-template <bool CA, bool CB> OPX_HD OPX_INLINE void mim(Acc &s, const M &a, const M &b, int r, int q) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int x = CA ? 3 * k + r : 3 * r + k, y = CB ? 3 * q + k : 3 * k + q;
-        mac(s, CB ? neg(a.r[x]) : a.r[x], b.i[y]);
-        mac(s, CA ? neg(a.i[x]) : a.i[x], b.r[y]);
-    }
-}
-template <bool CA, bool CB> OPX_HD OPX_INLINE void mmul(M &c, const M &a, const M &b) {
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            Acc s = acc0(), t = acc0();
-            mre<CA, CB>(s, a, b, r, q);
-            mim<CA, CB>(t, a, b, r, q);
-            c.r[3 * r + q] = pack(s);
-            c.i[3 * r + q] = pack(t);
-        }
-}
 // A row of a matrix.  The SU(3) kernels form products row by row, v -> v B, in a
 // loop over the three rows, with B's entries read from the link arrays as they are
 // used: a third of the code of whole matrix products (which overran the

@@ -121,12 +121,34 @@ static void su3(double w) {
             need(std::fabs(val(f.i[k]) - M.m[k / 3][k % 3].imag()) < TOL, what, (double)val(f.i[k]), (double)M.m[k / 3][k % 3].imag());
         }
     };
-    fx::M c;
-    fx::mmul<false, false>(c, a, b); cmp(c, mul(A[0], A[1]), "A B");
-    fx::mmul<true, false>(c, a, b); cmp(c, mul(adj(A[0]), A[1]), "A* B");
-    fx::mmul<false, true>(c, a, b); cmp(c, mul(A[0], adj(A[1])), "A B*");
+    // products row by row: row r of A or (dag) A^dagger times B or B^dagger
+    auto entries = [](const fx::M &m) { return [&m](int k, fx::Fx &re, fx::Fx &im) { re = m.r[k]; im = m.i[k]; }; };
+    auto row = [](const fx::M &m, int r, bool dag) {
+        fx::Row v;
+        for (int k = 0; k < 3; k++) {
+            const int x = dag ? 3 * k + r : 3 * r + k;
+            v.r[k] = m.r[x];
+            v.i[k] = dag ? fx::neg(m.i[x]) : m.i[x];
+        }
+        return v;
+    };
+    fx::M c, d, f;
     fx::i64 S[18] = {};
-    for (int k = 0; k < 4; k++) { if (k & 1) fx::macc<true, false>(S, a, b); else fx::macc<false, true>(S, a, b); }
+    for (int r = 0; r < 3; r++) {
+        const fx::Row ab = fx::rmul<false>(row(a, r, false), entries(b)), db = fx::rmul<false>(row(a, r, true), entries(b)),
+                      bd = fx::rmul<true>(row(a, r, false), entries(b));
+        for (int q = 0; q < 3; q++) {
+            c.r[3 * r + q] = ab.r[q]; c.i[3 * r + q] = ab.i[q];
+            d.r[3 * r + q] = db.r[q]; d.i[3 * r + q] = db.i[q];
+            f.r[3 * r + q] = bd.r[q]; f.i[3 * r + q] = bd.i[q];
+        }
+        fx::i64 T[6] = {};
+        for (int k = 0; k < 4; k++) { if (k & 1) fx::racc<false>(T, row(a, r, true), entries(b)); else fx::racc<true>(T, row(a, r, false), entries(b)); }
+        for (int q = 0; q < 3; q++) { S[3 * r + q] = T[q]; S[9 + 3 * r + q] = T[3 + q]; }
+    }
+    cmp(c, mul(A[0], A[1]), "A B");
+    cmp(d, mul(adj(A[0]), A[1]), "A* B");
+    cmp(f, mul(A[0], adj(A[1])), "A B*");
     const Mat<3> P = mul(adj(A[0]), A[1]), Q = mul(A[0], adj(A[1]));
     for (int k = 0; k < 9; k++) {
         const C r = (Wide)2 * (P.m[k / 3][k % 3] + Q.m[k / 3][k % 3]);
@@ -135,8 +157,19 @@ static void su3(double w) {
         fx::entry(c, 9 + k) = fx::quarter(S[9 + k]);
     }
     // proj of A times the quarter of that sum
-    fx::i64 p[8];
-    fx::mproj<false, false>(p, a, c);
+    fx::i64 p[9] = {};
+    for (int r = 0; r < 3; r++) {
+        const fx::Row v = row(a, r, false);
+        fx::i64 re[3], im[3];
+        for (int q = 0; q < 3; q++) {
+            fx::Acc x = fx::acc0v(), y = fx::acc0v();
+            fx::rterm<false>(x, y, v, entries(c), q);
+            re[q] = fx::value(x);
+            im[q] = fx::value(y);
+        }
+        fx::proj_row(p, r, re, im);
+    }
+    p[7] = fx::proj_eighth(p);
     Mat<3> R = {};
     for (int i = 0; i < 3; i++) for (int j = 0; j < 3; j++) R.m[i][j] = (P.m[i][j] + Q.m[i][j]) / (Wide)2;
     R = mul(A[0], R);
