@@ -11,7 +11,7 @@
 //       combined by one block in a fixed order, so results are deterministic.
 //   k_bulk_partial_su2f : the same for SU(2) FP32
 //   k_bulk_partial_fx  : the same for FP64 storage with the group products in
-//       fixed point (fixed.cuh), four threads a site
+//       fixed point (fixed.cuh), three warps for 32 sites
 //   k_energy_density   : EnergyDensity.ComponentComputation (EnergyDensity.java:119-166)
 //   k_projected_energy : ProjectedEnergyDensity.EnergyDensityComputation (:114-179)
 //   k_gauss_field      : Grid.getGaussConstraint (Grid.java:944-968) at every cell

@@ -726,7 +726,6 @@ __device__ __forceinline__ void update_link_pair(int i, const float *__restrict_
     }
 }
 
-// The three links of the two sites
 // L2 prefetch of the warp's E lines (3 links x 8 components x the two 32-site
 // halves from sa of lane 0), which the thread reads only after its staple sums:
 // their DRAM latency then overlaps the staples (0.5 % per 128^3 step, 2 % per step
@@ -743,6 +742,7 @@ __device__ __forceinline__ void prefetch_e_pair(const float *E, const Lat &L, I 
     }
 }
 
+// The three links of the two sites
 template <typename I, bool HAS_J, bool REUNIT, bool MEAS = false>
 __device__ __forceinline__ void update_site_pair(const float *__restrict__ U, float *__restrict__ E,
                                                  const float *__restrict__ J, float *__restrict__ Unext,
