@@ -13,6 +13,7 @@
 
 #include <cstdlib>
 
+#include "fixed.cuh"
 #include "internal.h"
 
 using namespace opx;
@@ -176,7 +177,8 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     if (ok && cudaMallocHost((void **)&c.red_host, sizeof(double) * 16) != cudaSuccess) ok = false;
     if (ok && (cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess)) ok = false;
     // without room for the fixed-point links the handle works all the same, in FP64 products
-    if (ok && c.fixed_kernel && (cudaMalloc(&c.fx_U, nU * 8) != cudaSuccess || cudaMalloc(&c.fx_Unext, nU * 8) != cudaSuccess)) {
+    const size_t fxb = fx::fixed_links_bytes(V, c.ng);
+    if (ok && c.fixed_kernel && (cudaMalloc(&c.fx_U, fxb) != cudaSuccess || cudaMalloc(&c.fx_Unext, fxb) != cudaSuccess)) {
         cudaGetLastError();
         if (c.fx_U) cudaFree(c.fx_U);
         c.fx_U = c.fx_Unext = nullptr;

@@ -44,6 +44,8 @@ struct Acc {
 constexpr int LINK_BAD = (int)0x80000000;     // h of a link's first entry when it is not usable here
 constexpr float LINK_TOL = 1.0f / 256.0f;     // largest |U^dagger U - 1| entry of a usable link
 constexpr int WEAK_H = 1 << 23;               // 2^-7 in units of 2^-30
+constexpr int SMALL_H = 1 << 16;              // 2^-14: a small component in the update (leapfrog_fx.cuh)
+constexpr int TINY_T = 1023 + 47;             // the exponent of 2^-14 in the exponential's argument, times 2^61
 constexpr i64 HALF30 = 1LL << 29, ONE30 = 1LL << 30;
 
 // the start of a sum that pack() ends (rounded, and offset for the split) and
@@ -92,6 +94,8 @@ OPX_HD OPX_INLINE double of_bits(i64 b) {
     return x;
 #endif
 }
+// x == 0 (an FP64 comparison would take the FP64 pipe)
+OPX_HD OPX_INLINE bool is_zero(double x) { return (bits_of(x) << 1) == 0; }
 OPX_HD OPX_INLINE int exponent_of(double x) { return (int)(bits_of(x) >> 52) & 0x7ff; }
 
 // x 2^61 rounded to nearest (ties away), for |x| < 2 (fx_of: 2 - 2^-30); integer operations only
@@ -467,7 +471,8 @@ template <int NC> OPX_HD OPX_INLINE typename LinkOf<NC>::T link_of(const double 
     return m;
 }
 
-// Whether the link lies within 2^-7 of the identity without being it
+// The largest entry off the identity (a bound within a factor of two, units of 2^-30; zero for
+// the identity): below WEAK_H, the link lies within 2^-7 of it
 OPX_HD OPX_INLINE int offdiag(const Q &q) { return absor(absor(absor(0, q.e[1]), q.e[2]), q.e[3]); }
 OPX_HD OPX_INLINE int offdiag(const M &m) {
     int o = absor(absor(absor(0, m.i[0]), m.i[4]), m.i[8]);
@@ -479,7 +484,18 @@ OPX_HD OPX_INLINE int offdiag(const M &m) {
 
 #ifdef __CUDACC__
 // Fixed-point links in global memory: the layout of the FP64 links, an entry's
-// eight bytes holding (l, h)
+// eight bytes holding (l, h).  SU(3) links have a word of flags each behind them,
+// [3][sites padded to 32]: what the update asks of every link of a stencil before it
+// forms a product (45 loads a thread from the entries themselves).  A bit per entry
+// off the identity (flag_bit): below 2^-14, and (ZERO_SHIFT) exactly zero as a double.
+constexpr unsigned SMALL_MASK = 0x7fff, LINK_WEAK = 1u << 30, FLAG_BAD = 1u << 31;
+constexpr int ZERO_SHIFT = 15;
+// entries 1, 2, 3, 5, 6, 7 (real), 9 .. 17 (imaginary) to bits 0 .. 14
+__host__ __device__ constexpr int flag_bit(int c) { return c >= 9 ? c - 3 : (c > 4 ? c - 2 : c - 1); }
+// bytes of an array of fixed-point links
+__host__ __device__ inline size_t fixed_links_bytes(long V, int ng) {
+    return (size_t)link_elems(V, ng) * 8 + (ng == 18 ? (size_t)link_blocks(V) * 32 * 3 * sizeof(unsigned) : 0);
+}
 template <int NC, typename I> struct FxLinks;
 template <typename I> struct FxLinks<2, I> {
     const int2 *p;
@@ -522,6 +538,10 @@ struct FxEntries {
 template <typename I> struct FxLinks<3, I> {
     const int2 *p;
     I V;
+    __device__ __forceinline__ unsigned flags(int d, I s) const {
+        const I n = ((V + 31) >> 5) << 5;
+        return __ldg(reinterpret_cast<const unsigned *>(p + 54 * n) + ((I)d * n + s));
+    }
     __device__ __forceinline__ FxEntries at(int d, I s) const { return FxEntries{p + link_offset_t<I>(V, 18, d, 0, s)}; }
     __device__ __forceinline__ M load(int d, I s) const {
         const int2 *b = p + link_offset_t<I>(V, 18, d, 0, s);
@@ -564,6 +584,20 @@ __device__ __forceinline__ void fixed_link(const R *U, int2 *out, I V, int d, I 
             const Fx x = entry(m, c);
             out[o + 32 * c] = make_int2(x.l, x.h);
         }
+        unsigned flags = entry(m, 0).h == LINK_BAD ? FLAG_BAD : 0u;
+        int all = 0;
+#pragma unroll
+        for (int c = 1; c < NG; c++) {
+            if (c == 4 || c == 8) continue;
+            const int h = abs(entry(m, c).h);
+            const unsigned bit = 1u << flag_bit(c);
+            all |= h;
+            if (h < SMALL_H) flags |= bit;
+            if (is_zero(u[c])) flags |= bit << ZERO_SHIFT;
+        }
+        if (all < WEAK_H) flags |= LINK_WEAK;
+        const I n = ((V + 31) >> 5) << 5;
+        reinterpret_cast<unsigned *>(out + 54 * n)[(I)d * n + s] = flags;
     }
 }
 

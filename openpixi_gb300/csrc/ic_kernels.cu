@@ -396,7 +396,7 @@ template <int NC, typename R> struct Cg {
     bool begin(double *mu_out, double stop, int maxit) {
         const long V = c.L.V, ns = V * c.na;
         const bool own = sizeof(R) == 8 && (const void *)U == c.U && c.fixed_kernel;
-        const size_t links = own ? 0 : (size_t)link_elems(V, c.ng) * 8;
+        const size_t links = own ? 0 : fx::fixed_links_bytes(V, c.ng);
         const size_t n = sizeof(double) * (size_t)(2 * ns + (mu_out ? 0 : ns) + 3 * ns) + links + sizeof(double) * 2 * MAX_BLOCKS + 256;
         if (cudaMalloc((void **)&arena, n + 256) != cudaSuccess || cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) != cudaSuccess) {

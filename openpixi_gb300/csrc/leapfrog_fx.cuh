@@ -7,10 +7,20 @@
 // staple planes need one factor 1/a_j^2 (equal spacings).
 //
 // update_link returns false, having written nothing, where a link it needs is
-// not usable in fixed point or where the link itself (SU(2): and the site's other
-// two, whose nine entries together are hardly ever all small by chance) lies
-// closer to the identity than 2^-7 in every entry (fixed.cuh: there the FP64
-// product is the more exact one); the caller then makes the FP64 update.
+// not usable in fixed point or where FP64 products are the more exact ones; the
+// caller then makes the FP64 update.  The latter is a matter of each colour
+// component: a product here is exact to 2^-61 of one, an FP64 product to 2^-53 of
+// the component's own size, so a component that is small in all links of a
+// stencil would lose its digits here.  A component (SU(3): an entry off the
+// identity) counts as small where it is below 2^-14 in all three links of the site;
+// all count as small where the site's links (SU(3): the link) are within 2^-7 of
+// the identity.  Small components that are exactly zero in the whole stencil stay
+// exactly zero here, so Abelian fields and vacuum keep the fixed-point form (the
+// product with an exponential whose argument has such a component, below 2^-14
+// but not zero, is FP64); any other small component is refused.  Components just
+// above the line keep 14 digits.  The line is as low as that because one warp that takes
+// the FP64 products by chance makes the whole grid wait (SU(3) 40^3 0.130 ms, with
+// 2^-10 0.181): at a width of 0.05 it is one link in 10^7 (SU(2): 10^8).
 //
 // Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.291 ms
 // a step, 128^3 2.014 -> 0.575, SU(3) 64^3 2.99 -> 0.492 ms (the FP64 pipe before);
@@ -31,7 +41,7 @@ namespace opx {
 namespace fx {
 
 // Unext of one link from its new E where qexp / mexp refuses (a large or
-// non-finite dt E): the FP64 exponential and product
+// non-finite dt E) or a component would lose digits: the FP64 exponential and product
 template <int NC, typename I>
 __device__ __forceinline__ void link_update_f64(const double *__restrict__ U, double *__restrict__ Un, const Lat &L, I s, int i,
                                              const double *e) {
@@ -42,9 +52,73 @@ __device__ __forceinline__ void link_update_f64(const double *__restrict__ U, do
     Unp.store(i, s, G::mul(G::expi(v), Up.load(i, s)));
 }
 
+// Bit a: component a + 1 of the three links of a site is small
+__device__ __forceinline__ int small_components(const Q &u0, const Q &u1, const Q &u2) {
+    int m[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) m[a] = abs(u0.e[1 + a].h) | abs(u1.e[1 + a].h) | abs(u2.e[1 + a].h);
+    const int all = m[0] | m[1] | m[2];
+    if (min(min(m[0], m[1]), m[2]) >= SMALL_H && all >= WEAK_H) return 0;
+    return all < WEAK_H ? 7 : (m[0] < SMALL_H ? 1 : 0) | (m[1] < SMALL_H ? 2 : 0) | (m[2] < SMALL_H ? 4 : 0);
+}
+// Whether the components of the mask are exactly zero in every link of the staples
+// of the site's three links (own, one step forward or back, and diagonal: 24 links).
+// From the doubles: the fixed-point form rounds what is below 2^-62 away
+template <typename I>
+__device__ __noinline__ bool zero_in_stencil(const double *U, const Lat &L, I s, int mask) {
+    const LinkPlanes<SU2<double>, double, I> Up{const_cast<double *>(U), (I)L.V};
+    auto zero = [&](int d, I t) {
+        const Q2<double> q = Up.load(d, t);
+        return (!(mask & 1) || is_zero(q.e[1])) && (!(mask & 2) || is_zero(q.e[2])) && (!(mask & 4) || is_zero(q.e[3]));
+    };
+    for (int d = 0; d < 3; d++)
+        if (!zero(d, s)) return false;
+    int x[3];
+    site_coords<I>(L, s, x);
+    const Deltas<I> D = deltas<I>(L, x);
+#pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+        const I mj = s + D.b(j);
+        if (!zero(j, mj)) return false;
+#pragma unroll 1
+        for (int ii = 1; ii < 3; ii++) {
+            const int i = j + ii >= 3 ? j + ii - 3 : j + ii;
+            if (!zero(i, mj) || !zero(i, s + D.f(j)) || !zero(j, s + D.f(i) + D.b(j))) return false;
+        }
+    }
+    return true;
+}
+// Whether a small component, zero in U, is to come out of exp(-i dt E) U with the
+// digits that FP64 gives it
+__device__ __forceinline__ bool tiny(double t) { return !is_zero(t) && exponent_of(t) < TINY_T; }
+__device__ __forceinline__ bool tiny_component(int small, const double *t) {
+    return small && (((small & 1) && tiny(t[0])) || ((small & 2) && tiny(t[1])) || ((small & 4) && tiny(t[2])));
+}
+// SU(3), small: a bit per entry (flag_bit).  H = -dt E^a lambda_a / 2 of the exponential:
+// i H has t_0, t_3, t_5 in its off-diagonal imaginary parts, t_1, t_4, t_6 in the real
+// ones, t_7 +- t_2 and -2 t_7 on the diagonal
+__device__ __forceinline__ bool tiny_entry(unsigned small, const double *t) {
+    if (!small) return false;
+    bool refuse = false;
+    auto see = [&](int c, int d, double h) {  // entries c and d of U, h of H
+        const unsigned both = 1u << flag_bit(c) | 1u << flag_bit(d);
+        refuse = refuse || ((small & both) == both && tiny(h));
+    };
+    see(10, 12, t[0]);
+    see(1, 3, t[1]);
+    see(11, 15, t[3]);
+    see(2, 6, t[4]);
+    see(14, 16, t[5]);
+    see(5, 7, t[6]);
+    see(9, 9, t[7] + t[2]);
+    see(13, 13, t[7] - t[2]);
+    see(17, 17, t[7]);
+    return refuse;
+}
+
 // SU(2): E and Unext of one link from its staple sum S (units of 2^-60, without 1/a^2)
 template <bool HAS_J, typename I>
-__device__ __forceinline__ void finish_link(const Q &Ui, const i64 *S, const double *__restrict__ U, double *__restrict__ E,
+__device__ __forceinline__ void finish_link(int small, const Q &Ui, const i64 *S, const double *__restrict__ U, double *__restrict__ E,
                                             const double *__restrict__ J, double *__restrict__ Unext, const Lat &L, I s, int i) {
     const AlgPlanes<3, double, I> Ep{E, (I)L.V}, Jp{const_cast<double *>(J), (I)L.V};
     const LinkPlanes<SU2<double>, double, I> Un{Unext, (I)L.V};
@@ -72,7 +146,7 @@ __device__ __forceinline__ void finish_link(const Q &Ui, const i64 *S, const dou
 #pragma unroll
     for (int a = 0; a < 3; a++) t[a] = kv * e[a];
     Q X;
-    if (qexp(t, X)) {
+    if (!tiny_component(small, t) && qexp(t, X)) {
         Q2<double> V;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -136,7 +210,8 @@ __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double 
     const Q Ui = W.load(i, s);
     const int j1 = i == 2 ? 0 : i + 1, j2 = i == 0 ? 2 : i - 1;
     const Q Uj1 = W.load(j1, s), Uj2 = W.load(j2, s);
-    if ((offdiag(Ui) | offdiag(Uj1) | offdiag(Uj2)) < WEAK_H) return false;
+    const int small = small_components(Ui, Uj1, Uj2);
+    if (small && !zero_in_stencil<I>(U, L, s, small)) return false;
     int x[3];
     site_coords<I>(L, s, x);
     const Deltas<I> D = deltas<I>(L, x);
@@ -156,7 +231,7 @@ __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double 
         qacc<true, false>(S, qmul<false, false>(load(i, s + bj), load(j, pi + bj)), load(j, s + bj));
     }
     if (worst == LINK_BAD) return false;
-    finish_link<HAS_J, I>(Ui, S, U, E, J, Unext, L, s, i);
+    finish_link<HAS_J, I>(small, Ui, S, U, E, J, Unext, L, s, i);
     return true;
 }
 
@@ -169,21 +244,22 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
     site_coords<I>(L, s, x);
     const Deltas<I> D = deltas<I>(L, x);
     const I pi = s + D.f(i);
-    int worst = 0;
-    auto see = [&](int d, I t) { worst = min(worst, __ldg(W.p + link_offset_t<I>(W.V, 18, d, 0, t)).y); };
-    see(i, s);
+    const int j1 = i == 2 ? 0 : i + 1, j2 = i == 0 ? 2 : i - 1;
+    const unsigned own = W.flags(i, s), u1 = W.flags(j1, s), u2 = W.flags(j2, s);
+    unsigned any = own | u1 | u2, every = own & u1 & u2;
+    const unsigned small = own & LINK_WEAK ? SMALL_MASK : every & SMALL_MASK;
 #pragma unroll
-    for (int jj = 1; jj < 3; jj++) {
-        const int j = i + jj >= 3 ? i + jj - 3 : i + jj;
+    for (int jj = 0; jj < 2; jj++) {
+        const int j = jj ? j2 : j1;
         const I bj = D.b(j);
-        see(j, s);
-        see(j, pi);
-        see(i, s + D.f(j));
-        see(i, s + bj);
-        see(j, s + bj);
-        see(j, pi + bj);
+        const unsigned f[5] = {W.flags(j, pi), W.flags(i, s + D.f(j)), W.flags(i, s + bj), W.flags(j, s + bj), W.flags(j, pi + bj)};
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            any |= f[k];
+            every &= f[k];
+        }
     }
-    if (worst == LINK_BAD || offdiag(W.load(i, s)) < WEAK_H) return false;
+    if ((any & FLAG_BAD) || (small & ~(every >> ZERO_SHIFT))) return false;
     const AlgPlanes<8, double, I> Ep{E, (I)L.V}, Jp{const_cast<double *>(J), (I)L.V};
     const LinkPlanes<SU3<double>, double, I> Un{Unext, (I)L.V};
     const double kdt = L.dt * L.inva2[0] * 0x1p-58, kv = L.dt * -0x1p60;
@@ -246,7 +322,7 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
     for (int a = 0; a < 7; a++) t[a] = kv * e[a];
     t[7] = kv * 0.57735026918962576451 * e[7];
     M X;
-    if (mexp(t, X)) {
+    if (!tiny_entry(small, t) && mexp(t, X)) {
         M3<double> V;
 #pragma unroll
         for (int r = 0; r < 3; r++) {
