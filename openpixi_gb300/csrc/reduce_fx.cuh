@@ -8,20 +8,20 @@
 namespace opx {
 namespace fx {
 
-template <int NC>
-__device__ __forceinline__ double plane_b2_f64(const double *__restrict__ U, const Lat &L, long s, const int *x, int d) {
+// In FP64, calls as in leapfrog_fx.cuh (SU(2): the last product's three components and
+// one factor for their squares)
+template <int NC, typename I>
+__device__ __noinline__ double plane_b2_f64(const double *__restrict__ U, const Lat &L, I s, I sj, I sk, int j, int k, double f) {
     using G = typename GroupOf<NC, double>::T;
-    const Nbr nb = neighbours(L, s, x);
-    const LinkPlanes<G, double> Up{const_cast<double *>(U), L.V};
-    const int j = d == 2 ? 0 : d + 1, k = d == 0 ? 2 : d - 1;
-    const long pj = pick3(nb.fwd[0], nb.fwd[1], nb.fwd[2], j), pk = pick3(nb.fwd[0], nb.fwd[1], nb.fwd[2], k);
-    auto P = G::mul_adj(G::mul_adj(G::mul(Up.load(j, s), Up.load(k, pj)), Up.load(j, pk)), Up.load(k, s));
-    double b[G::NA];
-    G::proj(P, b);
-    const double f = LatR<double>::bfac(L, d);
-#pragma unroll
-    for (int a = 0; a < G::NA; a++) b[a] *= f;
-    return sqr<double, G::NA>(b);
+    const LinkPlanes<G, double, I> Up{const_cast<double *>(U), (I)L.V};
+    const auto P = G::mul_adj(G::mul_adj(G::mul(Up.load(j, s), Up.load(k, sj)), Up.load(j, sk)), Up.load(k, s));
+    if constexpr (NC == 2) {
+        return (P.e[1] * P.e[1] + P.e[2] * P.e[2] + P.e[3] * P.e[3]) * (4.0 * (f * f));
+    } else {
+        double b[G::NA];
+        G::proj(P, b);
+        return sqr<double, G::NA>(b) * (f * f);
+    }
 }
 
 __device__ __forceinline__ double proj_square(const Q &A, const Q &B) {  // |proj(A B^dagger)|^2
@@ -40,20 +40,23 @@ template <typename I>
 __device__ __forceinline__ double plane_b2(const FxLinks<2, I> W, const double *__restrict__ U, const Lat &L, I s, const int *x,
                                            const Deltas<I> &D, int d) {
     const int j = d == 2 ? 0 : d + 1, k = d == 0 ? 2 : d - 1;
-    const Q Uj = W.load(j, s), Uk = W.load(k, s), A = W.load(k, s + D.f(j)), B = W.load(j, s + D.f(k));
-    if ((offdiag(Uj) | offdiag(Uk)) < WEAK_H || min(min(Uj.e[0].h, Uk.e[0].h), min(A.e[0].h, B.e[0].h)) == LINK_BAD)
-        return plane_b2_f64<2>(U, L, (long)s, x, d);
+    const I sj = s + D.f(j), sk = s + D.f(k);
     const double f = LatR<double>::bfac(L, d);
+    const Q Uj = W.load(j, s), Uk = W.load(k, s), A = W.load(k, sj), B = W.load(j, sk);
+    if ((offdiag(Uj) | offdiag(Uk)) < WEAK_H || min(min(Uj.e[0].h, Uk.e[0].h), min(A.e[0].h, B.e[0].h)) == LINK_BAD)
+        return plane_b2_f64<2, I>(U, L, s, sj, sk, j, k, f);
     return proj_square(qmul<false, true>(qmul<false, false>(Uj, A), B), Uk) * (f * f);
 }
 template <typename I>
 __device__ __forceinline__ double plane_b2(const FxLinks<3, I> W, const double *__restrict__ U, const Lat &L, I s, const int *x,
                                            const Deltas<I> &D, int d) {
     const int j = d == 2 ? 0 : d + 1, k = d == 0 ? 2 : d - 1;
-    const FxEntries Uj = W.at(j, s), Uk = W.at(k, s), A = W.at(k, s + D.f(j)), B = W.at(j, s + D.f(k));
+    const I sj = s + D.f(j), sk = s + D.f(k);
+    const double f = LatR<double>::bfac(L, d);
+    const FxEntries Uj = W.at(j, s), Uk = W.at(k, s), A = W.at(k, sj), B = W.at(j, sk);
     if ((offdiag(W.load(j, s)) | offdiag(W.load(k, s))) < WEAK_H ||
         min(min(Uj.mark(), Uk.mark()), min(A.mark(), B.mark())) == LINK_BAD)
-        return plane_b2_f64<3>(U, L, (long)s, x, d);
+        return plane_b2_f64<3, I>(U, L, s, sj, sk, j, k, f);
     i64 x9[9];
 #pragma unroll
     for (int a = 0; a < 9; a++) x9[a] = 0;
@@ -77,7 +80,6 @@ __device__ __forceinline__ double plane_b2(const FxLinks<3, I> W, const double *
         const double v = (double)x9[a];
         b2 = fma(v, v, b2);
     }
-    const double f = LatR<double>::bfac(L, d);
     return b2 * 0x1p-122 * (f * f);
 }
 

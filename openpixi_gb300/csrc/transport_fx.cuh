@@ -104,21 +104,29 @@ __device__ __forceinline__ double component(const Scaled<8> &t, int a) {
     return a == 7 ? (double)t.v[7] * 0.57735026918962576451 : (double)t.v[a];
 }
 
+// The same in FP64 (calls, as in leapfrog_fx.cuh).  SU(2): with a pure quaternion X the first
+// product has no scalar terms of X, and of the second three components are wanted: G::act without
+// its products with zero and its halves (24 instead of 34 operations)
 template <int NC, bool FWD, typename R>
-__device__ __forceinline__ void transport_f64(const R *__restrict__ U, const Lat &L, long s, int i, const double *x, double *t) {
+__device__ __noinline__ void transport_f64(const R *__restrict__ U, const Lat &L, long s, int i, const double *x, double *t) {
     using G = typename GroupOf<NC, double>::T;
     using GR = typename GroupOf<NC, R>::T;
     const auto u = LinkPlanes<GR, R>{const_cast<R *>(U), L.V}.load(i, s);
-    typename G::M g;
     if constexpr (NC == 2) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) g.e[c] = (double)u.e[c];
+        const double q = FWD ? -1.0 : 1.0, u0 = (double)u.e[0], u1 = q * (double)u.e[1], u2 = q * (double)u.e[2], u3 = q * (double)u.e[3];
+        // A = X V, t = V^dagger A, V = U or (FWD) its adjoint
+        const double a0 = -(x[0] * u1 + x[1] * u2 + x[2] * u3), a1 = x[0] * u0 - x[1] * u3 + x[2] * u2;
+        const double a2 = x[1] * u0 - x[2] * u1 + x[0] * u3, a3 = x[2] * u0 - x[0] * u2 + x[1] * u1;
+        t[0] = u0 * a1 - u1 * a0 + u2 * a3 - u3 * a2;
+        t[1] = u0 * a2 - u2 * a0 + u3 * a1 - u1 * a3;
+        t[2] = u0 * a3 - u3 * a0 + u1 * a2 - u2 * a1;
     } else {
+        typename G::M g;
 #pragma unroll
         for (int c = 0; c < 9; c++) { g.r[c] = (double)u.r[c]; g.i[c] = (double)u.i[c]; }
+        if constexpr (FWD) G::act(x, g, t);
+        else G::act(x, G::adj(g), t);
     }
-    if constexpr (FWD) G::act(x, g, t);
-    else G::act(x, G::adj(g), t);
 }
 
 // Whether a link's transport is formed in fixed point
