@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <map>
 #include <numeric>
 #include <string>
@@ -185,13 +186,13 @@ __global__ void k_batch_links(const BEvent<R> *__restrict__ ev, int nev, int cur
 constexpr int BATCH_RED_CHUNKS = 16;
 
 template <int NC, typename R>
-__global__ void __launch_bounds__(256) k_batch_bulk(const BEvent<R> *__restrict__ ev, int cur,
+__global__ void __launch_bounds__(256) k_batch_bulk(const BEvent<R> *__restrict__ ev, int cur, int fixed,
                                                     double *__restrict__ part) {
     const int q = blockIdx.y;
     const BEvent<R> &e = ev[q];
     KSum acc[NQ];
     bulk_accumulate<NC, R>(e.B[cur], e.B[cur ^ 1], e.E, nullptr, nullptr, e.L, acc,
-                           (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+                           (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x, fixed != 0);
     int qq;
     KSum v = block_reduce<NQ>(acc, qq);
     if (qq >= 0) {
@@ -237,6 +238,7 @@ struct Batch {
     double *staging = nullptr;
     std::string err;
     long launches = 0;
+    bool fp64_only = false;   // OPX_FP64_ONLY=1 at creation: no fixed-point products (internal.h)
     bool int_offsets = true;  // every event's link and E offsets fit in 32 bits
 };
 
@@ -456,6 +458,7 @@ int opx_batch_create(int ncolors, int nevents, const int *dims, const double *a,
     b.ng = ncolors == 3 ? 18 : 4;
     b.na = ncolors == 3 ? 8 : 3;
     b.prec = precision;
+    b.fp64_only = std::getenv("OPX_FP64_ONLY") != nullptr;
     b.nev = nevents;
     b.dt = dt;
     b.g = g;
@@ -749,11 +752,11 @@ int opx_batch_reduce(opx_batch *h, opx_observables *out) {
     Batch &b = h->b;
     dim3 grid(BATCH_RED_CHUNKS, b.nev);
     if (b.nc == 2) {
-        if (b.prec == OPX_F64) k_batch_bulk<2, double><<<grid, 256, 0, b.stream>>>((const BEvent<double> *)b.ev_dev, b.cur, b.red_part);
-        else k_batch_bulk<2, float><<<grid, 256, 0, b.stream>>>((const BEvent<float> *)b.ev_dev, b.cur, b.red_part);
+        if (b.prec == OPX_F64) k_batch_bulk<2, double><<<grid, 256, 0, b.stream>>>((const BEvent<double> *)b.ev_dev, b.cur, b.fp64_only ? 0 : 1, b.red_part);
+        else k_batch_bulk<2, float><<<grid, 256, 0, b.stream>>>((const BEvent<float> *)b.ev_dev, b.cur, b.fp64_only ? 0 : 1, b.red_part);
     } else {
-        if (b.prec == OPX_F64) k_batch_bulk<3, double><<<grid, 256, 0, b.stream>>>((const BEvent<double> *)b.ev_dev, b.cur, b.red_part);
-        else k_batch_bulk<3, float><<<grid, 256, 0, b.stream>>>((const BEvent<float> *)b.ev_dev, b.cur, b.red_part);
+        if (b.prec == OPX_F64) k_batch_bulk<3, double><<<grid, 256, 0, b.stream>>>((const BEvent<double> *)b.ev_dev, b.cur, b.fp64_only ? 0 : 1, b.red_part);
+        else k_batch_bulk<3, float><<<grid, 256, 0, b.stream>>>((const BEvent<float> *)b.ev_dev, b.cur, b.fp64_only ? 0 : 1, b.red_part);
     }
     k_batch_bulk_final<<<grid_for((long)b.nev * NQ, 256), 256, 0, b.stream>>>(b.red_part, b.nev, b.red_out);
     b.launches += 2;

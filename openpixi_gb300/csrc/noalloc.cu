@@ -26,6 +26,7 @@
 // that resets a device must not call this entry point on that device again.
 // Unlike opx_reduce, non-finite field values are not turned into an error
 // status; they reach the record as NaN or Inf, and the caller checks it.
+#include <cstdlib>
 #include <mutex>
 
 #include "internal.h"
@@ -42,11 +43,11 @@ static __device__ __align__(256) double g_noalloc_partials[OPX_NOALLOC_BLOCKS * 
 template <int NC, typename R>
 __global__ void __launch_bounds__(256) k_noalloc_partial(const R *__restrict__ U, const R *__restrict__ Unext,
                                                          const R *__restrict__ E, const R *__restrict__ rho,
-                                                         const uint8_t *__restrict__ eval, Lat L,
+                                                         const uint8_t *__restrict__ eval, Lat L, int fixed,
                                                          double *__restrict__ part) {
     KSum acc[NQ];
     bulk_accumulate<NC, R>(U, Unext, E, rho, eval, L, acc, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                           (long)gridDim.x * blockDim.x);
+                           (long)gridDim.x * blockDim.x, fixed != 0);
     int q;
     KSum v = block_reduce<NQ>(acc, q);
     if (q >= 0) {
@@ -102,11 +103,11 @@ static int noalloc_scratch(double **out) {
 }
 
 template <int NC, typename R>
-static void noalloc_launch(const Lat &L, const void *U, const void *Unext, const void *E, const void *rho,
+static void noalloc_launch(const Lat &L, int fixed, const void *U, const void *Unext, const void *E, const void *rho,
                            const uint8_t *eval, double *part, int nblocks, opx_observables *out,
                            cudaStream_t st) {
     k_noalloc_partial<NC, R><<<nblocks, 256, 0, st>>>((const R *)U, (const R *)Unext, (const R *)E,
-                                                      (const R *)rho, eval, L, part);
+                                                      (const R *)rho, eval, L, fixed, part);
     k_noalloc_final<<<1, 32, 0, st>>>(part, nblocks, (double)L.V, out);
 }
 
@@ -133,16 +134,19 @@ extern "C" int opx_reduce_noalloc(int ncolors, int precision, const int *dims, c
     int rc = noalloc_scratch(&part);
     if (rc) return rc;
     const Lat L = make_lat(dims, a, 1.0, g);
+    // the products of a handle made under the same environment (a handle that works without
+    // its fixed-point links for lack of memory forms them in FP64 all the same)
+    const int fixed = std::getenv("OPX_FP64_ONLY") == nullptr;
     const int nblocks = (int)std::min<long>((V + 255) / 256, OPX_NOALLOC_BLOCKS);
     cudaStream_t st = (cudaStream_t)stream;
     // an error left pending by earlier work of the caller is neither reported nor cleared here
     const cudaError_t pending = cudaPeekAtLastError();
     if (ncolors == 2) {
-        if (precision == OPX_F64) noalloc_launch<2, double>(L, U, Unext, E, rho, eval, part, nblocks, out_device, st);
-        else noalloc_launch<2, float>(L, U, Unext, E, rho, eval, part, nblocks, out_device, st);
+        if (precision == OPX_F64) noalloc_launch<2, double>(L, fixed, U, Unext, E, rho, eval, part, nblocks, out_device, st);
+        else noalloc_launch<2, float>(L, 0, U, Unext, E, rho, eval, part, nblocks, out_device, st);
     } else {
-        if (precision == OPX_F64) noalloc_launch<3, double>(L, U, Unext, E, rho, eval, part, nblocks, out_device, st);
-        else noalloc_launch<3, float>(L, U, Unext, E, rho, eval, part, nblocks, out_device, st);
+        if (precision == OPX_F64) noalloc_launch<3, double>(L, fixed, U, Unext, E, rho, eval, part, nblocks, out_device, st);
+        else noalloc_launch<3, float>(L, 0, U, Unext, E, rho, eval, part, nblocks, out_device, st);
     }
     const cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess && e != pending) {

@@ -68,12 +68,12 @@ __device__ __forceinline__ double sqr(const R *x) {
 // GaussLaw/TotalChargeSquared, physics/measurements/FieldMeasurements.java:68-231).
 // Runs of 32 sites are summed plainly in FP64 and folded into the compensated
 // sums, so the error stays at the compensated level while the FP64 work per
-// site is one addition per column.
+// site is one addition per column.  fixed (FP64 storage): Gauss transports in fixed point.
 template <int NC, typename R>
 __device__ __forceinline__ void bulk_accumulate(const R *__restrict__ U, const R *__restrict__ Unext,
                                                 const R *__restrict__ E, const R *__restrict__ rho,
                                                 const uint8_t *__restrict__ eval, const Lat &L, KSum *acc,
-                                                long first, long stride) {
+                                                long first, long stride, bool fixed) {
     using G = typename GroupOf<NC, R>::T;
     constexpr int NA = G::NA;
     const LinkPlanes<G, R> Up{const_cast<R *>(U), L.V}, Unp{const_cast<R *>(Unext), L.V};
@@ -104,8 +104,9 @@ __device__ __forceinline__ void bulk_accumulate(const R *__restrict__ U, const R
         }
         R gs[NA];
         if constexpr (sizeof(R) == 8) {
-            // the transports of opx_reduce (k_bulk_partial_fx), bit for bit
-            if (L.inva2[0] == L.inva2[1] && L.inva2[1] == L.inva2[2]) {
+            // fixed: the transports of opx_reduce (k_bulk_partial_fx), bit for bit, where the
+            // spacings are equal; otherwise those of its FP64 form
+            if (fixed && L.inva2[0] == L.inva2[1] && L.inva2[1] == L.inva2[2]) {
 #pragma unroll
                 for (int a = 0; a < NA; a++) gs[a] = 0.0;
 #pragma unroll 1
