@@ -399,12 +399,16 @@ namespace {
 // Device buffers of one call: get() hands out offsets, take() makes the one
 // allocation and at() the pointers (a gradient's fifty allocations and frees took 3 ms)
 struct DevBuf {
+    Ctx &c;
     char *base = nullptr;
     size_t bytes = 0;
     bool ok = true;
+    explicit DevBuf(Ctx &c_) : c(c_) {}
+    DevBuf(const DevBuf &) = delete;
+    DevBuf &operator=(const DevBuf &) = delete;
     template <typename T> T *get(size_t n) {
         void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) { ok = false; cudaGetLastError(); return nullptr; }
+        if (dev_malloc(c, &p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) { ok = false; return nullptr; }
         ptrs.push_back(p);
         return (T *)p;
     }
@@ -414,7 +418,7 @@ struct DevBuf {
         return o;
     }
     bool take() {
-        if (cudaMalloc((void **)&base, std::max<size_t>(bytes, 256)) != cudaSuccess) { ok = false; base = nullptr; cudaGetLastError(); }
+        if (dev_malloc(c, &base, std::max<size_t>(bytes, 256)) != cudaSuccess) ok = false;
         return ok;
     }
     template <typename T> T *at(size_t o) const { return (T *)(base + o); }
@@ -524,7 +528,7 @@ int input_direction(Ctx &c, const double *U64, const double *dE, const double *d
     cudaMemcpyAsync(dev, t.data(), nE * 8, cudaMemcpyHostToDevice, c.stream);
     cudaStreamSynchronize(c.stream);
     if (!drho) return OPX_OK;
-    DevBuf B;
+    DevBuf B(c);
     double *r = B.get<double>(nr), *mu = B.get<double>(nr);
     if (!B.ok) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
     std::vector<double> tr(nr);
@@ -540,7 +544,7 @@ int input_direction(Ctx &c, const double *U64, const double *dE, const double *d
 int objective_value_impl(Ctx &c, const ObjArgs &ar, int nsteps, const double *dE, const double *drho, double h,
                          double *J, const char *where) {
     const long V = c.L.V, nU = link_elems(V, 4), nE = V * 9;
-    DevBuf B;
+    DevBuf B(c);
     double *U0 = B.get<double>(nU), *Wa = B.get<double>(nU), *Wb = B.get<double>(nU), *E = B.get<double>(nE);
     double *dEd = B.get<double>(nE), *part = B.get<double>(8 * 304), *out4 = B.get<double>(4);
     if (!B.ok) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
@@ -562,7 +566,7 @@ int objective_value_impl(Ctx &c, const ObjArgs &ar, int nsteps, const double *dE
 int objective_tangent_impl(Ctx &c, const ObjArgs &ar, int nsteps, const double *dE, const double *drho, double *J,
                            double *dJ, const char *where) {
     const long V = c.L.V, nU = link_elems(V, 4), nE = V * 9;
-    DevBuf B;
+    DevBuf B(c);
     double *U0 = B.get<double>(nU), *E0 = B.get<double>(nE), *dEd = B.get<double>(nE);
     Dual *Ud = B.get<Dual>(nU), *Wa = B.get<Dual>(nU), *Wb = B.get<Dual>(nU), *Ed = B.get<Dual>(nE);
     double *part = B.get<double>(8 * 304), *out4 = B.get<double>(4);
@@ -596,7 +600,7 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
     // strides in bytes, whole lines (E's 72 V bytes alone would misalign the links after them)
     const size_t bU = (size_t)nU * 8, bE = ((size_t)nE * 8 + 255) & ~size_t(255);
     const int fixed = !c.fp64_only && c.L.inva2[0] == c.L.inva2[1] && c.L.inva2[1] == c.L.inva2[2];
-    DevBuf B;
+    DevBuf B(c);
     // forward in the handle's precision, its links in fixed point beside them (FP64)
     const size_t oWra = B.reserve(nU * rs), oWrb = B.reserve(nU * rs), oEr = B.reserve(nE * rs), oFa = B.reserve(bU), oFb = B.reserve(bU);
     const size_t oU64 = B.reserve(bU), oE64 = B.reserve(bE), oCk = B.reserve(nseg * (bU + bE)), oSeg = B.reserve((size_t)ckpt * (2 * bU + bE));

@@ -98,6 +98,30 @@ static void release(Ctx &c) {
     if (c.stream) cudaStreamDestroy(c.stream);
 }
 
+// Gives the fixed-point links back: the handle goes on with FP64 products
+bool opx::drop_fixed_links(Ctx &c) {
+    if (!c.fx_U) return false;
+    cudaStreamSynchronize(c.stream);
+    cudaFree(c.fx_U);
+    cudaFree(c.fx_Unext);
+    c.fx_U = c.fx_Unext = nullptr;
+    c.fixed_kernel = false;
+    c.links_changed();
+    return true;
+}
+cudaError_t opx::dev_malloc_bytes(Ctx &c, void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (drop_fixed_links(c)) e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+    }
+    return e;
+}
+
 // The device address of a page-locked host buffer of n doubles (cudaMallocHost
 // or cudaHostRegister memory, both ends mapped at one offset), or null for
 // pageable memory.  The conversion kernels read and write page-locked buffers
@@ -176,7 +200,9 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     al((void **)&c.status, sizeof(unsigned));
     if (ok && cudaMallocHost((void **)&c.red_host, sizeof(double) * 16) != cudaSuccess) ok = false;
     if (ok && (cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess)) ok = false;
-    // without room for the fixed-point links the handle works all the same, in FP64 products
+    // without room for the fixed-point links the handle works all the same, in FP64 products,
+    // and what it allocates later may have theirs (dev_malloc).  Other handles' allocations
+    // find that much less: 192 B a site for SU(2), 876 for SU(3)
     const size_t fxb = fx::fixed_links_bytes(V, c.ng);
     if (ok && c.fixed_kernel && (cudaMalloc(&c.fx_U, fxb) != cudaSuccess || cudaMalloc(&c.fx_Unext, fxb) != cudaSuccess)) {
         cudaGetLastError();
@@ -220,7 +246,7 @@ static int ensure_staging(Ctx &c, size_t ndoubles) {
     if (c.staging) cudaFree(c.staging);
     c.staging = nullptr;
     c.staging_len = 0;
-    if (cudaMalloc(&c.staging, ndoubles * sizeof(double)) != cudaSuccess) {
+    if (dev_malloc(c, &c.staging, ndoubles * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         c.err = "staging buffer: out of device memory";
         return OPX_ERR_NOMEM;
@@ -313,7 +339,7 @@ static int set_mask(Ctx &c, uint8_t **dst, const uint8_t *mask, size_t count, co
         return OPX_OK;
     }
     if (count != (size_t)c.L.V) { c.err = std::string(where) + ": count must equal the number of cells"; return OPX_ERR_INVALID; }
-    if (!*dst && cudaMalloc((void **)dst, c.L.V) != cudaSuccess) { cudaGetLastError(); c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
+    if (!*dst && dev_malloc(c, dst, c.L.V) != cudaSuccess) { cudaGetLastError(); c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
     cudaError_t e = cudaMemcpyAsync(*dst, mask, c.L.V, cudaMemcpyHostToDevice, c.stream);
     if (e != cudaSuccess) return cuda_fail(c, where, e);
     return sync_check(c, where);
@@ -541,7 +567,7 @@ static bool ensure_rows(Ctx &c, long n) {
     if (c.meas_host) cudaFreeHost(c.meas_host);
     c.meas_rows = c.meas_host = nullptr;
     c.meas_rows_cap = 0;
-    if (cudaMalloc((void **)&c.meas_rows, sizeof(double) * n) != cudaSuccess || cudaMallocHost((void **)&c.meas_host, sizeof(double) * n) != cudaSuccess)
+    if (dev_malloc(c, &c.meas_rows, sizeof(double) * n) != cudaSuccess || cudaMallocHost((void **)&c.meas_host, sizeof(double) * n) != cudaSuccess)
         return false;
     c.meas_rows_cap = n;
     return true;
@@ -550,10 +576,10 @@ static bool ensure_rows(Ctx &c, long n) {
 static int ensure_measure_buffers(Ctx &c, int nsteps) {
     const size_t nE = (size_t)c.L.V * 3 * c.na;
     bool ok = true;
-    if (!c.E_alt) ok = cudaMalloc(&c.E_alt, nE * c.rsize) == cudaSuccess;
+    if (!c.E_alt) ok = dev_malloc(c, &c.E_alt, nE * c.rsize) == cudaSuccess;
     for (void **w : {&c.W_in, &c.W_out})
         if (ok && !*w) {
-            ok = cudaMalloc(w, nE * c.rsize) == cudaSuccess;
+            ok = dev_malloc(c, w, nE * c.rsize) == cudaSuccess;
             if (ok) cudaMemsetAsync(*w, 0, nE * c.rsize, c.stream);  // the first step's Gauss term is unused
         }
     if (ok && !c.meas_part) {
@@ -561,7 +587,7 @@ static int ensure_measure_buffers(Ctx &c, int nsteps) {
         // with one launch per chunk of steps
         const size_t per_step = sizeof(double) * MEAS_ROW * measured_parts(c);
         c.meas_chunk = (int)std::max<size_t>(1, std::min<size_t>(64, ((size_t)64 << 20) / per_step));
-        ok = cudaMalloc((void **)&c.meas_part, per_step * c.meas_chunk) == cudaSuccess;
+        ok = dev_malloc(c, &c.meas_part, per_step * c.meas_chunk) == cudaSuccess;
         if (!ok) c.meas_chunk = 0;
     }
     ok = ok && ensure_rows(c, 8L * nsteps);
@@ -914,7 +940,7 @@ int opx_super_upload(opx_ctx *ctx, int orientation, long n, long base, const dou
     const int nar = c.na_ref;
     const size_t tot = (size_t)ppc * n * nar;
     if (tot) {
-        if (cudaMalloc(&G.Q, sizeof(double) * tot) != cudaSuccess) {
+        if (dev_malloc(c, &G.Q, sizeof(double) * tot) != cudaSuccess) {
             cudaGetLastError();
             c.err = "opx_super_upload: out of device memory";
             return OPX_ERR_NOMEM;

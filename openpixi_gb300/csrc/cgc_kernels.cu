@@ -545,7 +545,7 @@ static int cgc_nucleus(Ctx &c, const opx_mv_nucleus &nu, std::vector<double> &pp
     cufftDoubleComplex *f = nullptr;
     const size_t nU = (size_t)link_elems(V, c.ng);
     bool ok = true;
-    auto al = [&](void **p, size_t b) { if (ok && cudaMalloc(p, b) != cudaSuccess) { ok = false; *p = nullptr; } };
+    auto al = [&](void **p, size_t b) { if (ok && dev_malloc(c, p, b) != cudaSuccess) { ok = false; *p = nullptr; } };
     al((void **)&rho, sizeof(double) * NA * V);
     al((void **)&phi, sizeof(double) * NA * V);
     al((void **)&f, sizeof(cufftDoubleComplex) * V);
@@ -562,8 +562,8 @@ static int cgc_nucleus(Ctx &c, const opx_mv_nucleus &nu, std::vector<double> &pp
     FFTPlan p3, p2;
     if (ok) {
         int dims3[3] = {n0, n1, n2}, dims2[2] = {n1, n2};
-        p3.make(3, dims3, 1, c.stream);
-        p2.make(2, dims2, n0, c.stream);
+        auto plans = [&]() { return p3.make(3, dims3, 1, c.stream) && p2.make(2, dims2, n0, c.stream); };
+        if (!plans() && drop_fixed_links(c)) plans();
     }
     if (!ok || !p3.ok || !p2.ok) {
         c.err = "opx_cgc_mv: out of device memory or cuFFT plan failure";
@@ -660,7 +660,7 @@ static int cgc_nucleus(Ctx &c, const opx_mv_nucleus &nu, std::vector<double> &pp
         if (ppc < 1) {
             c.err = "opx_cgc_mv_super: round(aL/dt) particles per cell must be >= 1";
             rc = OPX_ERR_INVALID;
-        } else if (n > 0 && cudaMalloc(&sg->Q, sizeof(double) * (size_t)ppc * nar * n) != cudaSuccess) {
+        } else if (n > 0 && dev_malloc(c, &sg->Q, sizeof(double) * (size_t)ppc * nar * n) != cudaSuccess) {
             cudaGetLastError();
             sg->Q = nullptr;
             c.err = "opx_cgc_mv_super: out of device memory";
@@ -686,8 +686,8 @@ static int cgc_nucleus(Ctx &c, const opx_mv_nucleus &nu, std::vector<double> &pp
         const int nar = c.na_ref, nz = zEnd - zStart + 1;
         const long np = (long)nz * ntr * ppc;
         double *d0 = nullptr, *d1 = nullptr, *dv = nullptr, *dq = nullptr;
-        bool ok2 = cudaMalloc(&d0, sizeof(double) * 3 * np) == cudaSuccess && cudaMalloc(&d1, sizeof(double) * 3 * np) == cudaSuccess &&
-                   cudaMalloc(&dv, sizeof(double) * 3 * np) == cudaSuccess && cudaMalloc(&dq, sizeof(double) * nar * np) == cudaSuccess;
+        bool ok2 = dev_malloc(c, &d0, sizeof(double) * 3 * np) == cudaSuccess && dev_malloc(c, &d1, sizeof(double) * 3 * np) == cudaSuccess &&
+                   dev_malloc(c, &dv, sizeof(double) * 3 * np) == cudaSuccess && dev_malloc(c, &dq, sizeof(double) * nar * np) == cudaSuccess;
         if (!ok2 || ppc < 1) {
             cudaGetLastError();
             c.err = ppc < 1 ? "opx_cgc_mv: round(aL/dt) particles per cell must be >= 1" : "opx_cgc_mv: out of device memory";
@@ -819,14 +819,14 @@ extern "C" int opx_cgc_wilson_lines(opx_ctx *ctx, int nucleus, double *tadpole, 
     double *part = nullptr;
     long long *cnt = nullptr;
     const size_t nout = 1 + (dipole ? (size_t)nb : 0);
-    bool ok = cudaMalloc(&dev, sizeof(double) * nout) == cudaSuccess;
+    bool ok = dev_malloc(c, &dev, sizeof(double) * nout) == cudaSuccess;
     const double a1 = c.L.a[1], a2 = c.L.a[2];
     const double ds = std::min(n1 * a1, n2 * a2) * 0.5 / (double)nb;
     const int B = 64;
     const size_t smem = (size_t)nb * B * (sizeof(double) + sizeof(long long));
     if (dipole && nb > 0) {
-        ok = ok && cudaMalloc(&part, sizeof(double) * ntr * nb) == cudaSuccess;
-        ok = ok && cudaMalloc(&cnt, sizeof(long long) * ntr * nb) == cudaSuccess;
+        ok = ok && dev_malloc(c, &part, sizeof(double) * ntr * nb) == cudaSuccess;
+        ok = ok && dev_malloc(c, &cnt, sizeof(long long) * ntr * nb) == cudaSuccess;
         if (smem > 200 * 1024) ok = false;
     }
     if (!ok) {

@@ -376,7 +376,7 @@ int cpic_alloc(Ctx &c, long n) {
     const long cap = n > 0 ? n : 1;
     const int nar = c.na_ref;
     bool ok = true;
-    auto al = [&](void **p, size_t bytes) { if (cudaMalloc(p, bytes) != cudaSuccess) { ok = false; *p = nullptr; } };
+    auto al = [&](void **p, size_t bytes) { if (dev_malloc(c, p, bytes) != cudaSuccess) { ok = false; *p = nullptr; } };
     al((void **)&P.pos0, sizeof(double) * 3 * cap);
     al((void **)&P.pos1, sizeof(double) * 3 * cap);
     al((void **)&P.vel, sizeof(double) * 3 * cap);

@@ -341,8 +341,8 @@ static int implicit_update_t(Ctx &c) {
     const long V = c.L.V;
     const size_t nU = (size_t)link_elems(V, c.ng) * sizeof(R), nE = (size_t)V * 3 * c.na * sizeof(R);
     if (!c.imp_Ua) {
-        if (cudaMalloc(&c.imp_Ua, nU) != cudaSuccess || cudaMalloc(&c.imp_Ub, nU) != cudaSuccess ||
-            cudaMalloc(&c.imp_E, nE) != cudaSuccess) {
+        if (dev_malloc(c, &c.imp_Ua, nU) != cudaSuccess || dev_malloc(c, &c.imp_Ub, nU) != cudaSuccess ||
+            dev_malloc(c, &c.imp_E, nE) != cudaSuccess) {
             cudaGetLastError();
             c.err = "implicit solver: out of device memory";
             return OPX_ERR_NOMEM;

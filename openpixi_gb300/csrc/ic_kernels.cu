@@ -124,7 +124,7 @@ int ic_init_random(Ctx &c, uint64_t seed, double sigma_a, double sigma_e) {
     double *U64 = nullptr, *E64 = nullptr;
     const bool f32 = c.prec == OPX_F32;
     if (f32) {
-        if (cudaMalloc(&U64, nU * 8) != cudaSuccess || cudaMalloc(&E64, nE * 8) != cudaSuccess) {
+        if (dev_malloc(c, &U64, nU * 8) != cudaSuccess || dev_malloc(c, &E64, nE * 8) != cudaSuccess) {
             cudaFree(U64);
             c.err = "opx_init_random: cannot allocate FP64 scratch";
             return OPX_ERR_NOMEM;
@@ -395,10 +395,23 @@ template <int NC, typename R> struct Cg {
     // mu_out: where the solution goes (null: a buffer of its own)
     bool begin(double *mu_out, double stop, int maxit) {
         const long V = c.L.V, ns = V * c.na;
-        const bool own = sizeof(R) == 8 && (const void *)U == c.U && c.fixed_kernel;
-        const size_t links = own ? 0 : fx::fixed_links_bytes(V, c.ng);
-        const size_t n = sizeof(double) * (size_t)(2 * ns + (mu_out ? 0 : ns) + 3 * ns) + links + sizeof(double) * 2 * MAX_BLOCKS + 256;
-        if (cudaMalloc((void **)&arena, n + 256) != cudaSuccess || cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
+        // with the handle's own fixed-point links the arena has none; without room for it
+        // these are given back
+        bool own = sizeof(R) == 8 && (const void *)U == c.U && c.fixed_kernel;
+        size_t links = 0;
+        auto take_arena = [&]() {
+            links = own ? 0 : fx::fixed_links_bytes(V, c.ng);
+            const size_t n = sizeof(double) * (size_t)(2 * ns + (mu_out ? 0 : ns) + 3 * ns) + links + sizeof(double) * 2 * MAX_BLOCKS + 512;
+            if (cudaMalloc((void **)&arena, n) == cudaSuccess) return true;
+            cudaGetLastError();
+            arena = nullptr;
+            return false;
+        };
+        if (!take_arena() && drop_fixed_links(c)) {
+            own = false;
+            take_arena();
+        }
+        if (!arena || cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
             return false;

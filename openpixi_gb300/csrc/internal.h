@@ -184,6 +184,11 @@ void launch_update_grid(Ctx &c, bool reunit);
 int launch_implicit_update(Ctx &c);  // ImplicitTYMSolver.step in place of launch_update_grid
 void launch_update_links(Ctx &c);
 void launch_reunit(Ctx &c, void *links);
+// cudaMalloc for what a call of the handle needs: where it fails, once more without the
+// handle's fixed-point links (no pointer to them is held across it)
+bool drop_fixed_links(Ctx &c);
+cudaError_t dev_malloc_bytes(Ctx &c, void **p, size_t bytes);
+template <typename T> inline cudaError_t dev_malloc(Ctx &c, T **p, size_t bytes) { return dev_malloc_bytes(c, (void **)p, bytes); }
 void ensure_fixed_links(Ctx &c, bool u, bool unext);  // fx_U / fx_Unext of the present links
 // the measured step (SU(3) FP32 paired form, FastTYMSolver, no current, no
 // masks, no particles): row[0..6] = E^2 of the new E [3] (x (g a_i)^-2),

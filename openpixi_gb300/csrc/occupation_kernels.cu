@@ -433,19 +433,20 @@ static int occupation_t(Ctx &c, const opx_occupation_options *opt, int max_iter,
     double *Ucm = nullptr, *Uncm = nullptr, *Ecm = nullptr;
     cufftDoubleComplex *F = nullptr;
     const int B = 256, nb = (int)std::min<long>(grid_for(Vm, B), 4L * 152);
-    bool ok = cudaMalloc(&Uc, sizeof(double) * nU) == cudaSuccess && cudaMalloc(&Unc, sizeof(double) * nU) == cudaSuccess &&
-              cudaMalloc(&Ec, sizeof(double) * 3 * NA * V) == cudaSuccess &&
-              cudaMalloc(&F, sizeof(cufftDoubleComplex) * std::max(6L * NA * V, (long)NA * Vm)) == cudaSuccess &&
-              cudaMalloc(&part, sizeof(double) * 2 * NA * nb) == cudaSuccess &&
-              (!n_out || cudaMalloc(&nd, sizeof(double) * NA * V) == cudaSuccess);
+    bool ok = dev_malloc(c, &Uc, sizeof(double) * nU) == cudaSuccess && dev_malloc(c, &Unc, sizeof(double) * nU) == cudaSuccess &&
+              dev_malloc(c, &Ec, sizeof(double) * 3 * NA * V) == cudaSuccess &&
+              dev_malloc(c, &F, sizeof(cufftDoubleComplex) * std::max(6L * NA * V, (long)NA * Vm)) == cudaSuccess &&
+              dev_malloc(c, &part, sizeof(double) * 2 * NA * nb) == cudaSuccess &&
+              (!n_out || dev_malloc(c, &nd, sizeof(double) * NA * V) == cudaSuccess);
     if (md >= 0)
-        ok = ok && cudaMalloc(&Ucm, sizeof(double) * nUm) == cudaSuccess &&
-             cudaMalloc(&Uncm, sizeof(double) * nUm) == cudaSuccess &&
-             cudaMalloc(&Ecm, sizeof(double) * 3 * NA * Vm) == cudaSuccess;
+        ok = ok && dev_malloc(c, &Ucm, sizeof(double) * nUm) == cudaSuccess &&
+             dev_malloc(c, &Uncm, sizeof(double) * nUm) == cudaSuccess &&
+             dev_malloc(c, &Ecm, sizeof(double) * 3 * NA * Vm) == cudaSuccess;
     int rc = OPX_OK;
     FFTPlan p3, p18;
     int dims[3] = {c.L.n[0], c.L.n[1], c.L.n[2]};
-    if (ok) ok = p3.make(3, dm, NA, c.stream) && p18.make(3, dims, 6 * NA, c.stream);
+    auto plans = [&]() { return p3.make(3, dm, NA, c.stream) && p18.make(3, dims, 6 * NA, c.stream); };
+    if (ok) ok = plans() || (drop_fixed_links(c) && plans());
     if (!ok) {
         cudaGetLastError();
         c.err = "opx_occupation_numbers: out of device memory or cuFFT plan failure";

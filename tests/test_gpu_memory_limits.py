@@ -1,0 +1,78 @@
+"""Calls that fit in the device's memory without the optional fixed-point copies of the
+FP64 links still run when those copies do not fit beside them: the gradient's stored
+steps, and what a handle allocates after its creation.
+
+A filler takes the device's memory but for the amount under test.  Kernels are loaded
+(a first call) before that."""
+import numpy as np
+import pytest
+
+import openpixi_gb300 as opx
+from openpixi_gb300 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+class Filler:
+    """Device memory but for `free` bytes and 12 MB at most (torch takes whole segments of
+    at least 10 MB)."""
+
+    def __init__(self, torch, free):
+        torch.cuda.empty_cache()
+        torch.cuda.synchronize()
+        self.torch, self.blocks = torch, []
+        while torch.cuda.mem_get_info()[0] - free >= 12 * MB:
+            n = min(torch.cuda.mem_get_info()[0] - free, 16 << 30)
+            self.blocks.append(torch.empty(int(n) // (2 * MB) * (2 * MB), dtype=torch.uint8, device="cuda"))
+
+    def release(self):
+        self.blocks = []
+        self.torch.cuda.empty_cache()
+
+
+def handle(nc, dims, sigma=0.1, prec=N.OPX_F64, **kw):
+    h = opx.Handle(nc, dims, dt=0.05, precision=prec, **kw)
+    h.init_random(3, sigma, sigma)
+    return h
+
+
+@pytest.mark.parametrize("nc", [2, 3])
+def test_handle_gives_its_fixed_links_back(native, nc):
+    """What is allocated after creation finds the memory of the fixed-point links."""
+    torch = pytest.importorskip("torch")
+    dims = (64, 64, 64)
+    v = 64 ** 3
+    ng, na = (4, 3) if nc == 2 else (18, 8)
+    warm, h, ref = (handle(nc, dims) for _ in range(3))
+    for x in (warm, h, ref):
+        x.initialize()
+    E = h.download(N.FIELD_E, layout=N.LAYOUT_GEN)
+    ref.step(3)
+    warm.set_field_solver(N.SOLVER_IMPLICIT, 1, 0.5)
+    warm.step(1)
+    warm.gauss_project(1e-20)
+    warm.close()
+    h.step(2)
+    # the projection's arena is six site vectors, less than the two copies of the links
+    arena = 6 * 8 * na * v
+    fill = Filler(torch, arena // 2)
+    try:
+        h.upload(N.FIELD_E, E, layout=N.LAYOUT_GEN)
+        it, g2 = h.gauss_project(1e-20)
+        assert g2 <= 1e-20
+        h.upload(N.FIELD_E, E, layout=N.LAYOUT_GEN)
+        h.step(1)
+        h.reduce()
+    finally:
+        fill.release()
+    h.upload(N.FIELD_U, ref.download(N.FIELD_U))
+    h.upload(N.FIELD_UNEXT, ref.download(N.FIELD_UNEXT))
+    h.upload(N.FIELD_E, ref.download(N.FIELD_E, layout=N.LAYOUT_GEN), layout=N.LAYOUT_GEN)
+    h.step(2), ref.step(2)
+    for f in (N.FIELD_UNEXT, N.FIELD_E):
+        x, y = h.download(f), ref.download(f)
+        assert np.abs(x - y).max() <= 1e-14 * np.abs(y).max()
+    a, b = h.reduce(), ref.reduce()
+    assert abs(a.e2_total + a.b2_total - b.e2_total - b.b2_total) <= 1e-13 * (b.e2_total + b.b2_total)
