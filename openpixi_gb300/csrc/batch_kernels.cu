@@ -695,7 +695,13 @@ int opx_batch_autotune(opx_batch *h, int steps, int *cluster_out, int *block_out
     Batch &b = h->b;
     // snapshot the fields: the trial runs advance the events
     char *snap = nullptr;
-    if (cudaMalloc(&snap, b.store_bytes) != cudaSuccess) { cudaGetLastError(); return batch_fail(b, "opx_batch_autotune: out of device memory", OPX_ERR_NOMEM); }
+    if (cudaMalloc(&snap, b.store_bytes) != cudaSuccess) {
+        // once more without the staging buffer, which the next pageable transfer allocates again
+        cudaGetLastError();
+        cudaFree(b.staging);
+        b.staging = nullptr;
+        if (cudaMalloc(&snap, b.store_bytes) != cudaSuccess) { cudaGetLastError(); return batch_fail(b, "opx_batch_autotune: out of device memory", OPX_ERR_NOMEM); }
+    }
     cudaMemcpyAsync(snap, b.store, b.store_bytes, cudaMemcpyDeviceToDevice, b.stream);
     const int cur0 = b.cur;
     const long steps0 = b.steps;

@@ -76,3 +76,22 @@ def test_handle_gives_its_fixed_links_back(native, nc):
         assert np.abs(x - y).max() <= 1e-14 * np.abs(y).max()
     a, b = h.reduce(), ref.reduce()
     assert abs(a.e2_total + a.b2_total - b.e2_total - b.b2_total) <= 1e-13 * (b.e2_total + b.b2_total)
+
+
+def test_batch_gives_its_staging_back(native):
+    """Autotune's copy of the fields finds the memory of the transfers' staging buffer."""
+    torch = pytest.importorskip("torch")
+    dims = (64, 64, 64)
+    v = 64 ** 3
+    b = opx.Batch(3, [dims], dt=0.05)
+    b.init_random([3], 0.1, 0.1)
+    b.initialize()
+    b.autotune(steps=1)
+    store, staging = v * (2 * 3 * 18 + 3 * 8) * 4, v * 3 * 18 * 8
+    U = b.download(0, N.FIELD_U)  # pageable: takes the staging buffer
+    fill = Filler(torch, store - staging // 2)
+    try:
+        b.autotune(steps=1)
+    finally:
+        fill.release()
+    assert np.array_equal(b.download(0, N.FIELD_U), U)
