@@ -417,8 +417,14 @@ struct DevBuf {
         bytes += (n + 255) & ~size_t(255);
         return o;
     }
-    bool take() {
-        if (dev_malloc(c, &base, std::max<size_t>(bytes, 256)) != cudaSuccess) ok = false;
+    // give: whether the handle's fixed-point links may go for it
+    bool take(bool give) {
+        const size_t n = std::max<size_t>(bytes, 256);
+        ok = (give ? dev_malloc(c, &base, n) : cudaMalloc((void **)&base, n)) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            base = nullptr;
+        }
         return ok;
     }
     template <typename T> T *at(size_t o) const { return (T *)(base + o); }
@@ -600,27 +606,43 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
     // strides in bytes, whole lines (E's 72 V bytes alone would misalign the links after them)
     const size_t bU = (size_t)nU * 8, bE = ((size_t)nE * 8 + 255) & ~size_t(255);
     const int fixed = !c.fp64_only && c.L.inva2[0] == c.L.inva2[1] && c.L.inva2[1] == c.L.inva2[2];
+    // Forward in the handle's precision; FP64 steps have their links in fixed point beside
+    // them.  KEEP keeps those of every step of a segment (264 instead of 168 B a site
+    // and step) for the reverse sweep; where that does not fit, REBUILD forms them again
+    // there from the stored links, the same values (64^3, 42 steps: 23.0 and 27.9 ms)
+    enum { KEEP, REBUILD } form = KEEP;
     DevBuf B(c);
-    // forward in the handle's precision, its links in fixed point beside them (FP64)
-    const size_t oWra = B.reserve(nU * rs), oWrb = B.reserve(nU * rs), oEr = B.reserve(nE * rs), oFa = B.reserve(bU), oFb = B.reserve(bU);
-    const size_t oU64 = B.reserve(bU), oE64 = B.reserve(bE), oCk = B.reserve(nseg * (bU + bE)), oSeg = B.reserve((size_t)ckpt * (2 * bU + bE));
-    const size_t oBar = B.reserve(2 * (bU + bE)), oWm = B.reserve(bU), oM = B.reserve(bE), oUown = B.reserve(bU);
-    const size_t oPart = B.reserve(8 * 8 * 304), oOut = B.reserve(32);
-    if (!B.take()) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
+    size_t oWra, oWrb, oEr, oFa, oFb, oU64, oE64, oCk, oSeg, oBar, oWm, oM, oUown, oPart, oOut, bSeg;
+    auto reserve = [&]() {
+        B.bytes = 0;
+        bSeg = bU + bE + (fixed && form == KEEP ? bU : 0);
+        oWra = B.reserve(nU * rs), oWrb = B.reserve(nU * rs), oEr = B.reserve(nE * rs);
+        oFa = oFb = 0;
+        if (fixed && (f64 || form == REBUILD)) oFa = B.reserve(bU), oFb = B.reserve(bU);
+        oU64 = B.reserve(bU), oE64 = B.reserve(bE), oCk = B.reserve(nseg * (bU + bE)), oSeg = B.reserve((size_t)ckpt * bSeg);
+        oBar = B.reserve(2 * (bU + bE)), oWm = B.reserve(bU), oM = B.reserve(bE), oUown = B.reserve(bU);
+        oPart = B.reserve(8 * 8 * 304), oOut = B.reserve(32);
+        return B.take(!fixed || form == REBUILD);
+    };
+    if (!reserve()) {
+        form = REBUILD;
+        if (!fixed || !reserve()) { c.err = std::string(where) + ": out of device memory"; return OPX_ERR_NOMEM; }
+    }
     double *U64 = B.at<double>(oU64), *E64 = B.at<double>(oE64), *part = B.at<double>(oPart), *out4 = B.at<double>(oOut);
     double *Wm_b = B.at<double>(oWm), *Mv = B.at<double>(oM), *Uown = B.at<double>(oUown);
     double *Wbar[2] = {B.at<double>(oBar), B.at<double>(oBar + bU)}, *Ebar[2] = {B.at<double>(oBar + 2 * bU), B.at<double>(oBar + 2 * bU + bE)};
     char *Er = B.at<char>(oEr);
     auto ckW = [&](int k) { return B.at<double>(oCk + k * (bU + bE)); };
     auto ckE = [&](int k) { return B.at<double>(oCk + k * (bU + bE) + bU); };
-    // W_{start + m} and E_{start + m} (m = 1 .. ckpt) of a segment, and the fixed-point form of W_{start + m - 1}
-    auto segW = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * (2 * bU + bE)); };
-    auto segE = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * (2 * bU + bE) + bU); };
-    auto segF = [&](int m) { return B.at<int2>(oSeg + (size_t)(m - 1) * (2 * bU + bE) + bU + bE); };
+    // W_{start + m} and E_{start + m} (m = 1 .. ckpt) of a segment, and the fixed-point form of
+    // W_{start + m - 1} (REBUILD: two buffers in turn)
+    auto segW = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * bSeg); };
+    auto segE = [&](int m) { return B.at<double>(oSeg + (size_t)(m - 1) * bSeg + bU); };
+    auto segF = [&](int m) { return form == REBUILD ? B.at<int2>(m & 1 ? oFa : oFb) : B.at<int2>(oSeg + (size_t)(m - 1) * bSeg + bU + bE); };
     widen_state(c, U64, E64);
     cudaMemcpyAsync(Er, c.E, nE * rs, cudaMemcpyDeviceToDevice, c.stream);
     const dim3 gs(grid_for(V, 128));
-    // one FP64 step from W (fixed point F) with E in place; Fn: W_{n+1} in fixed point
+    // one FP64 step from W (fixed point F) with E in place; Fn: W_{n+1} in fixed point (or null)
     auto to_fixed = [&](const double *W, int2 *F) {
         fx::k_fixed_links<2, double><<<dim3(gs.x, 3), 128, 0, c.stream>>>(W, F, c.L);
         c.launches++;
@@ -670,7 +692,7 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
         if (fixed) to_fixed(ckW(k), segF(1));
         for (int m = 1; m <= len; m++) {
             cudaMemcpyAsync(segE(m), m == 1 ? ckE(k) : segE(m - 1), nE * 8, cudaMemcpyDeviceToDevice, c.stream);
-            step64(segF(m), W_at(m - 1), segE(m), segW(m), m < len ? segF(m + 1) : Fc);
+            step64(segF(m), W_at(m - 1), segE(m), segW(m), m < len ? segF(m + 1) : nullptr);
         }
         if (k == nseg - 1) {
             double AB[2];
@@ -689,6 +711,7 @@ int objective_gradient_impl(Ctx &c, const ObjArgs &ar, int nsteps, int ckpt, int
         }
         for (int m = len; m >= 1; m--) {
             const int n = start + m;
+            if (fixed && form == REBUILD && m < len) to_fixed(W_at(m - 1), segF(m));
             if (c.int_offsets) {
                 k_adj_local<int><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), segE(m), Wbar[wb], Ebar[wb], c.L, fixed, Mv, Uown, Ebar[wb ^ 1]);
                 fx::k_adj_gather_fx<int><<<3 * gs.x, 128, 0, c.stream>>>(segF(m), W_at(m - 1), Mv, Uown, c.L, fixed, Wbar[wb ^ 1]);

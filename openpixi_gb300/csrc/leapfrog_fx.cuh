@@ -462,7 +462,7 @@ k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, dou
     if (!update_link<HAS_J, I>(FxLinks<NC, I>{Uf, (I)L.V}, U, E, J, Unext, L, s, i))
         update_link_f64<HAS_J, I>(LinkPlanes<typename GroupOf<NC, double>::T, double, I>{const_cast<double *>(U), (I)L.V}, E, J, Unext, L, s, i);
     // the new link in fixed point, from the double that was stored
-    fixed_link<NC, double, I>(Unext, Unf, (I)L.V, i, s);
+    if (Unf) fixed_link<NC, double, I>(Unext, Unf, (I)L.V, i, s);
 }
 
 }  // namespace fx

@@ -38,6 +38,46 @@ def handle(nc, dims, sigma=0.1, prec=N.OPX_F64, **kw):
     return h
 
 
+N_GRAD, STEPS = 64, 24
+V = N_GRAD ** 3
+LINKS, FIELDS = 96 * V, 72 * V  # bytes of one FP64 copy of the links and of E
+
+
+# with every step's fixed-point links 264 B a site and step, without 168 B: two margins
+# between the sum of either form's other buffers and the next form's
+@pytest.mark.parametrize("spare", [10, 4])
+def test_gradient_without_room_for_fixed_links(native, spare):
+    torch = pytest.importorskip("torch")
+    h = handle(2, (N_GRAD,) * 3)
+    J0, g0 = h.energy_gradient(STEPS, STEPS)
+    # checkpoint, cotangents, two of each field in flight, and `spare` arrays of links
+    need = (STEPS + 1) * (LINKS + FIELDS) + 2 * (LINKS + FIELDS) + 6 * LINKS + 3 * FIELDS + spare * LINKS // 2
+    fill = Filler(torch, need)
+    try:
+        J, g = h.energy_gradient(STEPS, STEPS)
+    finally:
+        fill.release()
+    # the same products, or FP64 ones where not even one more copy fits
+    assert abs(J - J0) <= 1e-13 * abs(J0)
+    assert np.abs(g - g0).max() <= 1e-12 * np.abs(g0).max()
+
+
+@pytest.mark.parametrize("kw", [dict(a=(1.0, 0.5, 1.0)), dict(prec=N.OPX_F32)])
+def test_gradient_reserves_what_it_uses(native, kw):
+    """Unequal spacings use no fixed-point links, an FP32 handle none of its own."""
+    torch = pytest.importorskip("torch")
+    h = handle(2, (N_GRAD,) * 3, **kw)
+    h.energy_gradient(STEPS, STEPS)
+    need = (STEPS + 1) * (LINKS + FIELDS) + 2 * (LINKS + FIELDS) + 6 * LINKS + 3 * FIELDS
+    if "prec" in kw:
+        need += 2 * LINKS
+    fill = Filler(torch, need)
+    try:
+        h.energy_gradient(STEPS, STEPS)
+    finally:
+        fill.release()
+
+
 @pytest.mark.parametrize("nc", [2, 3])
 def test_handle_gives_its_fixed_links_back(native, nc):
     """What is allocated after creation finds the memory of the fixed-point links."""
