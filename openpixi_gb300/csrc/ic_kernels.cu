@@ -14,6 +14,7 @@
 // draw the same A and E.
 #include <algorithm>
 
+#include "cg_loop.h"
 #include "internal.h"
 #include "ksum.cuh"
 #include "observables.cuh"
@@ -383,7 +384,7 @@ template <int NC, typename R> struct Cg {
     double *r = nullptr, *p = nullptr, *mu = nullptr, *t = nullptr, *part = nullptr;
     CgState *st = nullptr;
     unsigned *count = nullptr;
-    int blocks = 1, fixed = 1;
+    int blocks = 1, fixed = 1, maxit = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     static constexpr int MAX_BLOCKS = 4 * 152;  // resident at once
 
@@ -393,7 +394,8 @@ template <int NC, typename R> struct Cg {
         if (arena) cudaFree(arena);
     }
     // mu_out: where the solution goes (null: a buffer of its own)
-    bool begin(double *mu_out, double stop, int maxit) {
+    bool begin(double *mu_out, double stop, int maxit_) {
+        maxit = maxit_;
         const long V = c.L.V, ns = V * c.na;
         // with the handle's own fixed-point links the arena has none; without room for it
         // these are given back
@@ -443,12 +445,13 @@ template <int NC, typename R> struct Cg {
         cudaStreamSynchronize(c.stream);  // the pinned state is free again
         return true;
     }
-    // iterations until done; the final state
-    CgState iterate() {
+    // iterations until done; the first error of the runtime
+    cudaError_t iterate() {
         constexpr int STEPS = 8;
         CgState *h = (CgState *)c.red_host;
         const long ns = c.L.V * c.na;
-        for (int k = 0;; k++) {
+        cudaError_t err = cudaSuccess;
+        auto queue = [&](long k) {
             for (int j = 0; j < STEPS; j++) {
                 k_cg_direction<<<std::min(grid_for(ns, 256), 8 * 152), 256, 0, c.stream>>>(st, r, p, ns);
                 k_cg_gradient<NC, R, false><<<blocks, 96, 0, c.stream>>>(st, Uf, U, p, c.L, fixed, t, nullptr, part, count);
@@ -457,13 +460,14 @@ template <int NC, typename R> struct Cg {
             c.launches += 3 * STEPS;
             cudaMemcpyAsync((char *)h + 64 * (k & 1), st, sizeof(CgState), cudaMemcpyDeviceToHost, c.stream);
             cudaEventRecord(ev[k & 1], c.stream);
-            if (k == 0) continue;
-            const int o = (k & 1) ^ 1;  // the batch before this one
-            if (cudaEventSynchronize(ev[o]) != cudaSuccess) break;
-            const CgState *s = (const CgState *)((const char *)h + 64 * o);
-            if (s->done) break;
-        }
-        return read();
+            return (err = cudaGetLastError()) == cudaSuccess;
+        };
+        auto look = [&](long k) {
+            if ((err = cudaEventSynchronize(ev[k & 1])) != cudaSuccess) return CG_FAILED;
+            return ((const CgState *)((const char *)h + 64 * (k & 1)))->done ? CG_DONE : CG_GOES_ON;
+        };
+        cg_batches(std::max<long>(1, ((long)maxit + STEPS - 1) / STEPS), queue, look);
+        return err;
     }
     CgState read() {
         CgState *h = (CgState *)c.red_host;
@@ -481,14 +485,16 @@ template <int NC, typename R> int project_t(Ctx &c, double tol, int maxit, int *
     const R *rho = c.rho_nonzero ? (const R *)c.rho : nullptr;
     k_cg_divergence<NC, R, R, CG_BEGIN><<<cg.blocks, 96, 0, c.stream>>>(cg.st, cg.Uf, cg.U, (const R *)c.E, rho, c.L, cg.fixed, cg.r, cg.p, cg.mu,
                                                                         cg.part, cg.count);
-    const CgState s = cg.iterate();
+    cudaError_t e = cg.iterate();
+    const CgState s = cg.read();
+    if (e != cudaSuccess) { c.err = std::string("opx_gauss_project: ") + cudaGetErrorString(e); return OPX_ERR_CUDA; }
     // E <- E + divT mu, and the residual recomputed from the projected field
     k_cg_gradient<NC, R, true><<<cg.blocks, 96, 0, c.stream>>>(cg.st, cg.Uf, cg.U, cg.mu, c.L, cg.fixed, cg.t, (R *)c.E, cg.part, cg.count);
     k_cg_divergence<NC, R, double, CG_END><<<cg.blocks, 96, 0, c.stream>>>(cg.st, cg.Uf, cg.U, cg.t, rho, c.L, cg.fixed, nullptr, nullptr, nullptr,
                                                                            cg.part, cg.count);
     c.launches += 3;
     const double g2 = cg.read().pAp / V;
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (iters) *iters = s.it;
     if (final_g2) *final_g2 = g2;
     if (e != cudaSuccess) { c.err = std::string("opx_gauss_project: ") + cudaGetErrorString(e); return OPX_ERR_CUDA; }
@@ -500,8 +506,9 @@ template <int NC> int solve_t(Ctx &c, const double *U64, const double *b, double
     if (!cg.begin(x, tol_rel, maxit)) { c.err = "covariant Laplacian solve: out of device memory"; return OPX_ERR_NOMEM; }
     k_cg_start<<<cg.blocks, 96, 0, c.stream>>>(cg.st, b, c.L.V * c.na, cg.r, cg.p, cg.mu, cg.part, cg.count);
     c.launches++;
-    const CgState s = cg.iterate();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cg.iterate();
+    const CgState s = cg.read();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (iters) *iters = s.it;
     if (e != cudaSuccess) { c.err = std::string("covariant Laplacian solve: ") + cudaGetErrorString(e); return OPX_ERR_CUDA; }
     if (s.rr > s.stop && s.rr > 0) { c.err = "covariant Laplacian solve: no convergence"; return OPX_ERR_NUMERIC; }
