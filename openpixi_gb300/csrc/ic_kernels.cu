@@ -397,21 +397,28 @@ template <int NC, typename R> struct Cg {
     bool begin(double *mu_out, double stop, int maxit_) {
         maxit = maxit_;
         const long V = c.L.V, ns = V * c.na;
-        // with the handle's own fixed-point links the arena has none; without room for it
-        // these are given back
+        // With the handle's own fixed-point links the arena has none; without room for it
+        // these are given back, and without room for its own an FP64 solve goes without:
+        // the FP64 products of every link, Uf the doubles, which nothing then looks at (an FP32
+        // solve keeps its array, an FP64 one's size, in any case)
         bool own = sizeof(R) == 8 && (const void *)U == c.U && c.fixed_kernel;
         size_t links = 0;
         auto take_arena = [&]() {
-            links = own ? 0 : fx::fixed_links_bytes(V, c.ng);
+            links = own || (sizeof(R) == 8 && !fixed) ? 0 : fx::fixed_links_bytes(V, c.ng);
             const size_t n = sizeof(double) * (size_t)(2 * ns + (mu_out ? 0 : ns) + 3 * ns) + links + sizeof(double) * 2 * MAX_BLOCKS + 512;
             if (cudaMalloc((void **)&arena, n) == cudaSuccess) return true;
             cudaGetLastError();
             arena = nullptr;
             return false;
         };
-        if (!take_arena() && drop_fixed_links(c)) {
+        fixed = c.fp64_only ? 0 : 1;
+        if (!take_arena()) {
+            const bool given = drop_fixed_links(c);
             own = false;
-            take_arena();
+            if (!(given && take_arena()) && sizeof(R) == 8) {
+                fixed = 0;
+                take_arena();
+            }
         }
         if (!arena || cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) != cudaSuccess) {
@@ -428,10 +435,11 @@ template <int NC, typename R> struct Cg {
         part = (double *)take(16 * MAX_BLOCKS);
         st = (CgState *)take(sizeof(CgState));
         count = (unsigned *)take(sizeof(unsigned));
-        fixed = c.fp64_only ? 0 : 1;
         if (own) {
             ensure_fixed_links(c, true, false);
             Uf = (const int2 *)c.fx_U;
+        } else if (!links) {
+            Uf = (const int2 *)U;
         } else {
             fx::k_fixed_links<NC, R><<<dim3(grid_for(V, 128), 3), 128, 0, c.stream>>>(U, f, c.L);
             c.launches++;

@@ -135,3 +135,25 @@ def test_batch_gives_its_staging_back(native):
     finally:
         fill.release()
     assert np.array_equal(b.download(0, N.FIELD_U), U)
+
+
+@pytest.mark.parametrize("prec", [N.OPX_F32, N.OPX_F64])
+def test_charge_direction_without_room_for_fixed_links(native, prec):
+    """The covariant solve of a charge direction: six site vectors beside the run's own
+    buffers (three of links, two of E, two site vectors)."""
+    torch = pytest.importorskip("torch")
+    n = 96
+    v = n ** 3
+    h = handle(2, (n,) * 3, prec=prec)
+    drho = np.random.default_rng(5).normal(0, 0.1, (v, 3))
+    J0 = h.objective_value(2, drho=drho, h=0.5)
+    need = (3 * 96 + 2 * 72 + (2 + 6) * 24) * v + 4 * MB
+    if prec == N.OPX_F64:
+        need -= 2 * 96 * v  # the handle's own
+    fill = Filler(torch, need)
+    try:
+        J = h.objective_value(2, drho=drho, h=0.5)
+    finally:
+        fill.release()
+    # conjugate gradients to 1e-13 of the right side, either way
+    assert abs(J - J0) <= 1e-9 * abs(J0)
