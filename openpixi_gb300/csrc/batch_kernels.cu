@@ -135,13 +135,13 @@ template <> struct FlatBounds<2, float> { static constexpr int minb = 4; };
 
 template <int NC, typename R, typename I, bool REUNIT>
 __global__ void __launch_bounds__(256, FlatBounds<NC, R>::minb) k_batch_flat(const BEvent<R> *__restrict__ ev, const int *__restrict__ order,
-                                                    const int *__restrict__ bstart, int nev, int rd) {
+                                                    const int *__restrict__ bstart, int nev, int rd, int cold) {
     pdl_wait();
     const int q = flat_event(bstart, nev, (int)blockIdx.x);
     const BEvent<R> &e = ev[order[q]];
     const I s = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
     if (s >= (I)e.L.V) return;
-    if constexpr (NC == 2) update_site_su2_planes<R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s, (long)nev * e.L.V >= 500000);
+    if constexpr (NC == 2) update_site_su2_planes<R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s, cold != 0);
     else update_site<NC, R, false, REUNIT, I>(e.B[rd], e.E, nullptr, e.B[rd ^ 1], e.L, s);
 }
 
@@ -149,13 +149,13 @@ __global__ void __launch_bounds__(256, FlatBounds<NC, R>::minb) k_batch_flat(con
 template <typename I, bool REUNIT>
 __global__ void __launch_bounds__(128, 3) k_batch_flat_su3f(const BEvent<float> *__restrict__ ev,
                                                             const int *__restrict__ order,
-                                                            const int *__restrict__ bstart, int nev, int rd) {
+                                                            const int *__restrict__ bstart, int nev, int rd, int cold) {
     pdl_wait();
     const int q = flat_event(bstart, nev, (int)blockIdx.x);
     const BEvent<float> &e = ev[order[q]];
     const I t = (I)((int)blockIdx.x - bstart[q]) * (I)blockDim.x + (I)threadIdx.x;
     const I V = (I)e.L.V, sa = ((t >> 5) << 6) + (t & 31);
-    if ((long)nev * e.L.V >= 200000) prefetch_e_pair<I>(e.E, e.L, sa);  // 312 B a site: the batch is not held in L2
+    if (cold) prefetch_e_pair<I>(e.E, e.L, sa);
     if (sa >= V) return;
     I sb = sa + 32;
     const bool vb = sb < V;
@@ -345,10 +345,16 @@ static cudaError_t launch_flat(Batch &b, int nsteps, cudaStream_t st) {
     const BEvent<R> *ev = (const BEvent<R> *)b.ev_dev;
     const int *order = b.order_dev, *bstart = b.bstart_dev;
     int nev = b.nev;
+    // cold: the fields of all events (132 B a site for SU(2), 528 for SU(3)) do not stay in
+    // L2 from step to step, and E is worth a prefetch (100 SU(2) events of 16^3 and one of 64^3:
+    // 29.9 -> 28.5 us a step against the line at each event's own volume times the events)
+    long sites = 0;
+    for (auto &L : b.lats) sites += L.V;
+    int cold = sites >= (NC == 2 ? 500000 : 200000) ? 1 : 0;
     for (int k = 0; k < nsteps; k++) {
         const bool reunit = b.reunit_every > 0 && ((step0 + k + 1) % b.reunit_every) == 0;
         int rd = b.cur ^ ((k + 1) & 1);
-        void *args[] = {(void *)&ev, (void *)&order, (void *)&bstart, (void *)&nev, (void *)&rd};
+        void *args[] = {(void *)&ev, (void *)&order, (void *)&bstart, (void *)&nev, (void *)&rd, (void *)&cold};
         void *kf = b.int_offsets ? (reunit ? flat_kernel<NC, R, int, true>() : flat_kernel<NC, R, int, false>())
                                  : (reunit ? flat_kernel<NC, R, long, true>() : flat_kernel<NC, R, long, false>());
         // the steps overlap as in launch_pdl (in a captured graph too)
