@@ -125,8 +125,10 @@ cudaError_t opx::dev_malloc_bytes(Ctx &c, void **p, size_t bytes) {
 // The device address of a page-locked host buffer of n doubles (cudaMallocHost
 // or cudaHostRegister memory, both ends mapped at one offset), or null for
 // pageable memory.  The conversion kernels read and write page-locked buffers
-// directly over the host link; pageable ones go through the staging copy.
+// directly over the host link; pageable ones go through the staging copy, and so does a
+// buffer off the eight-byte grid, which a copy takes and a kernel's load of a double does not.
 double *opx::device_view(const void *host, size_t n) {
+    if ((uintptr_t)host % sizeof(double) != 0) return nullptr;
     cudaPointerAttributes a0, a1;
     const char *first = (const char *)host, *last = first + n * sizeof(double) - 1;
     if (cudaPointerGetAttributes(&a0, first) != cudaSuccess || cudaPointerGetAttributes(&a1, last) != cudaSuccess) {
