@@ -142,7 +142,7 @@ k_adj_local(const int2 *__restrict__ Wf, const double *__restrict__ Wprev, const
     for (int a = 0; a < 3; a++) eb[a] += -dt * vb[a];
     const double m[3] = {2 * dt * eb[0], 2 * dt * eb[1], 2 * dt * eb[2]};
     Q S;
-    if (!(fixed && fx::staple_sum_fx<I>(fx::FxLinks<2, I>{Wf, (I)L.V}, L, s, deltas<I>(L, x), i, S)))
+    if (!(fixed && fx::staple_sum_fx<I>(fx::FxLinks<2, I>{Wf, (I)L.V}, Wprev, L, s, deltas<I>(L, x), i, S)))
         S = staple_sum(LinkPlanes<G2, double>{const_cast<double *>(Wprev), L.V}, L, (long)s, x, i);
     qacc(own, fx::left_mul(m, qadj(S)));
     Mp.store(i, s, m);

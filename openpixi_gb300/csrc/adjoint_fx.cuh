@@ -30,14 +30,15 @@ __device__ __forceinline__ Qd right_mul(const Qd &q, const double *m) {
                m[1] * q.e[0] + m[2] * q.e[1] - m[0] * q.e[3], m[2] * q.e[0] + m[0] * q.e[2] - m[1] * q.e[1]}};
 }
 
-// The staple sum S_i(s) (with 1/a_j^2) of the links W, in doubles; false where a
-// link is not usable in fixed point or the link is within 2^-7 of the identity
+// The staple sum S_i(s) (with 1/a_j^2) of the links W, in doubles; false where the update
+// would refuse the link (leapfrog_fx.cuh)
 template <typename I>
-__device__ __forceinline__ bool staple_sum_fx(const FxLinks<2, I> W, const Lat &L, I s, const Deltas<I> &D, int i, Qd &S) {
+__device__ __forceinline__ bool staple_sum_fx(const FxLinks<2, I> W, const double *__restrict__ U, const Lat &L, I s, const Deltas<I> &D, int i, Qd &S) {
     const Q Ui = W.load(i, s);
     const int j1 = i == 2 ? 0 : i + 1, j2 = i == 0 ? 2 : i - 1;
     const Q Uj1 = W.load(j1, s), Uj2 = W.load(j2, s);
-    if ((offdiag(Ui) | offdiag(Uj1) | offdiag(Uj2)) < WEAK_H) return false;
+    const int small = small_components(Ui, Uj1, Uj2);
+    if (small && !zero_in_stencil<I>(U, L, s, small)) return false;
     int worst = min(min(Ui.e[0].h, Uj1.e[0].h), Uj2.e[0].h);
     auto load = [&](int d, I t) {
         const Q q = W.load(d, t);
@@ -92,9 +93,9 @@ k_adj_gather_fx(const int2 *__restrict__ Wf, const double *__restrict__ Wd, cons
     const LinkPlanes<G2d, double, I> Wp{const_cast<double *>(Wd), (I)L.V}, UO{const_cast<double *>(Uown), (I)L.V}, OUT{Wbar_prev, (I)L.V};
     const I ypk = y + D.f(k);
     Qd out = UO.load(k, y);
-    // the largest exponent of the M that enter
+    // the largest exponent of the M that enter, and their components that are not all zero
     int emax = 0, worst = 0;
-    bool any = false;
+    unsigned some[3] = {0u, 0u, 0u};
     auto see = [&](int d, I s) {
         double m[3];
         Mp.load_ro(d, s, m);
@@ -102,7 +103,7 @@ k_adj_gather_fx(const int2 *__restrict__ Wf, const double *__restrict__ Wd, cons
         for (int a = 0; a < 3; a++) {
             const int e = exponent_of(m[a]);
             emax = e > emax ? e : emax;
-            any = any || (bits_of(m[a]) << 1) != 0;
+            some[a] |= (unsigned)__double2loint(m[a]) | ((unsigned)__double2hiint(m[a]) << 1);
         }
     };
 #pragma unroll
@@ -116,11 +117,20 @@ k_adj_gather_fx(const int2 *__restrict__ Wf, const double *__restrict__ Wd, cons
         see(k, z);
         see(i, z + D.f(k));
     }
-    if (!any) {
+    if (!(some[0] | some[1] | some[2])) {
         OUT.store(k, y, out);
         return;
     }
     bool ok = fixed && emax >= 64 && emax < 0x7ff;
+    if (ok) {
+        // a component that is small in the links keeps its digits only if it is zero in all (as in
+        // the update; links near the identity lose none: M itself is of order one)
+        const int small = small_components<false>(W.load(0, y), W.load(1, y), W.load(2, y));
+        if (small) {
+            const int nonzero = (some[0] ? 1 : 0) | (some[1] ? 2 : 0) | (some[2] ? 4 : 0);
+            if ((small & nonzero) || !zero_in_stencil<I>(Wd, L, y, small)) ok = false;
+        }
+    }
     if (ok) {
         auto mval = [&](int d, I s, i64 *v) {  // below 1/4 in units of 2^-61
             double m[3];

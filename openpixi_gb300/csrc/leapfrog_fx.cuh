@@ -52,14 +52,16 @@ __device__ __noinline__ void link_update_f64(const double *__restrict__ U, doubl
     Unp.store(i, s, G::mul(G::expi(v), Up.load(i, s)));
 }
 
-// Bit a: component a + 1 of the three links of a site is small
-__device__ __forceinline__ int small_components(const Q &u0, const Q &u1, const Q &u2) {
+// Bit a: component a + 1 of the three links of a site is small; WEAK: all where the
+// links are within 2^-7 of the identity
+template <bool WEAK = true> __device__ __forceinline__ int small_components(const Q &u0, const Q &u1, const Q &u2) {
     int m[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) m[a] = abs(u0.e[1 + a].h) | abs(u1.e[1 + a].h) | abs(u2.e[1 + a].h);
     const int all = m[0] | m[1] | m[2];
-    if (min(min(m[0], m[1]), m[2]) >= SMALL_H && all >= WEAK_H) return 0;
-    return all < WEAK_H ? 7 : (m[0] < SMALL_H ? 1 : 0) | (m[1] < SMALL_H ? 2 : 0) | (m[2] < SMALL_H ? 4 : 0);
+    const bool weak = WEAK && all < WEAK_H;
+    if (min(min(m[0], m[1]), m[2]) >= SMALL_H && !weak) return 0;
+    return weak ? 7 : (m[0] < SMALL_H ? 1 : 0) | (m[1] < SMALL_H ? 2 : 0) | (m[2] < SMALL_H ? 4 : 0);
 }
 // Whether the components of the mask are exactly zero in every link of the staples
 // of the site's three links (own, one step forward or back, and diagonal: 24 links).

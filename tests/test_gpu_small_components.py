@@ -128,3 +128,28 @@ def test_vacuum_and_abelian_fields_stay_exact(native, monkeypatch, nc):
     # sites whose stencil is vacuum over both steps: planes 0 .. of the first half, away from its edges
     far = np.arange(V).reshape(DIMS)[2:DIMS[0] // 2 - 2].ravel()
     assert np.array_equal(ua[far], ub[far]) and np.array_equal(ea[far], eb[far])
+
+
+@pytest.mark.parametrize("eps", EPS)
+@pytest.mark.parametrize("form", [0, 1])
+def test_gradient_in_small_components(native, monkeypatch, form, eps):
+    """The gradient with respect to E is of the size of the field in each component (its
+    sums come in no fixed order: some tens of roundings more)."""
+    nc, big, small, _ = FORMS[form]
+    rng = np.random.default_rng(20 + form)
+    V = int(np.prod(DIMS))
+    A, E = (np.zeros((V, 3, 3)) for _ in range(2))
+    for X in (A, E):
+        X[..., big] = rng.normal(0, 0.15, (V, 3, len(big)))
+        X[..., small] = rng.normal(0, eps, (V, 3, len(small)))
+    out = []
+    for only in (True, False):
+        if only:
+            monkeypatch.setenv("OPX_FP64_ONLY", "1")
+        else:
+            monkeypatch.delenv("OPX_FP64_ONLY")
+        h = opx.Handle(nc, DIMS, precision=N.OPX_F64, dt=0.05)
+        h.upload(N.FIELD_U, links(nc, A))
+        h.upload(N.FIELD_E, E, layout=N.LAYOUT_GEN)
+        out.append(h.energy_gradient(6, 4, (2, 1, 3), (4, 4, 6))[1].reshape(V, 3, 3))
+    close(out[0], out[1], [big, small])
