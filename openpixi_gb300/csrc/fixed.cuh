@@ -556,6 +556,44 @@ template <typename I> struct FxLinks<3, I> {
     }
 };
 
+// The entries u of link (d, s) in fixed point into out
+template <int NC, typename I>
+__device__ __forceinline__ void write_fixed(const double *u, int2 *out, I V, int d, I s) {
+    constexpr int NG = LinkOf<NC>::NG;
+    const I o = link_offset_t<I>(V, NG, d, 0, s);
+    auto m = link_of<NC>(u);
+    if constexpr (NC == 2) {
+        int4 *q = reinterpret_cast<int4 *>(out + o);
+        q[0] = make_int4(m.e[0].l, m.e[0].h, m.e[1].l, m.e[1].h);
+        q[1] = make_int4(m.e[2].l, m.e[2].h, m.e[3].l, m.e[3].h);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NG; c++) {
+            const Fx x = entry(m, c);
+            out[o + 32 * c] = make_int2(x.l, x.h);
+        }
+        unsigned flags = entry(m, 0).h == LINK_BAD ? FLAG_BAD : 0u;
+        int all = 0, least = SMALL_H;
+#pragma unroll
+        for (int c = 1; c < NG; c++) {
+            if (c == 4 || c == 8) continue;
+            const int h = abs(entry(m, c).h);
+            all |= h;
+            least = min(least, h);
+        }
+        if (all < WEAK_H) flags |= LINK_WEAK;
+        if (least < SMALL_H) {  // hardly ever
+#pragma unroll
+            for (int c = 1; c < NG; c++) {
+                if (c == 4 || c == 8) continue;
+                const unsigned bit = 1u << flag_bit(c);
+                if (abs(entry(m, c).h) < SMALL_H) flags |= is_zero(u[c]) ? bit | bit << ZERO_SHIFT : bit;
+            }
+        }
+        const I n = ((V + 31) >> 5) << 5;
+        reinterpret_cast<unsigned *>(out + 54 * n)[(I)d * n + s] = flags;
+    }
+}
 // Link (d, s) of U (double, or float: widened) in fixed point into out
 template <int NC, typename R, typename I>
 __device__ __forceinline__ void fixed_link(const R *U, int2 *out, I V, int d, I s) {
@@ -573,32 +611,7 @@ __device__ __forceinline__ void fixed_link(const R *U, int2 *out, I V, int d, I 
 #pragma unroll
         for (int c = 0; c < NG; c++) u[c] = (double)U[o + 32 * c];
     }
-    auto m = link_of<NC>(u);
-    if constexpr (NC == 2) {
-        int4 *q = reinterpret_cast<int4 *>(out + o);
-        q[0] = make_int4(m.e[0].l, m.e[0].h, m.e[1].l, m.e[1].h);
-        q[1] = make_int4(m.e[2].l, m.e[2].h, m.e[3].l, m.e[3].h);
-    } else {
-#pragma unroll
-        for (int c = 0; c < NG; c++) {
-            const Fx x = entry(m, c);
-            out[o + 32 * c] = make_int2(x.l, x.h);
-        }
-        unsigned flags = entry(m, 0).h == LINK_BAD ? FLAG_BAD : 0u;
-        int all = 0;
-#pragma unroll
-        for (int c = 1; c < NG; c++) {
-            if (c == 4 || c == 8) continue;
-            const int h = abs(entry(m, c).h);
-            const unsigned bit = 1u << flag_bit(c);
-            all |= h;
-            if (h < SMALL_H) flags |= bit;
-            if (is_zero(u[c])) flags |= bit << ZERO_SHIFT;
-        }
-        if (all < WEAK_H) flags |= LINK_WEAK;
-        const I n = ((V + 31) >> 5) << 5;
-        reinterpret_cast<unsigned *>(out + 54 * n)[(I)d * n + s] = flags;
-    }
+    write_fixed<NC, I>(u, out, V, d, s);
 }
 
 // One link per thread (blockIdx.y its direction)

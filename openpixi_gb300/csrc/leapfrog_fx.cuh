@@ -121,7 +121,8 @@ __device__ __forceinline__ bool tiny_entry(unsigned small, const double *t) {
 // SU(2): E and Unext of one link from its staple sum S (units of 2^-60, without 1/a^2)
 template <bool HAS_J, typename I>
 __device__ __forceinline__ void finish_link(int small, const Q &Ui, const i64 *S, const double *__restrict__ U, double *__restrict__ E,
-                                            const double *__restrict__ J, double *__restrict__ Unext, const Lat &L, I s, int i) {
+                                            const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf,
+                                            const Lat &L, I s, int i) {
     const AlgPlanes<3, double, I> Ep{E, (I)L.V}, Jp{const_cast<double *>(J), (I)L.V};
     const LinkPlanes<SU2<double>, double, I> Un{Unext, (I)L.V};
     const double kdt = L.dt * L.inva2[0] * 0x1p-58, kv = L.dt * -0x1p60;
@@ -157,8 +158,10 @@ __device__ __forceinline__ void finish_link(int small, const Q &Ui, const i64 *S
             V.e[c] = double_of(value(p));
         }
         Un.store(i, s, V);
+        if (Unf) write_fixed<2, I>(V.e, Unf, (I)L.V, i, s);
     } else {
         link_update_f64<2, I>(U, Unext, L, s, i, e);
+        if (Unf) fixed_link<2, double, I>(Unext, Unf, (I)L.V, i, s);
     }
 }
 
@@ -308,7 +311,7 @@ __device__ __noinline__ void update_link_f64(const LinkPlanes<SU3<double>, doubl
 // SU(2), one link
 template <bool HAS_J, typename I>
 __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double *__restrict__ U, double *__restrict__ E,
-                                            const double *__restrict__ J, double *__restrict__ Unext, const Lat &L, I s, int i) {
+                                            const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf, const Lat &L, I s, int i) {
     const Q Ui = W.load(i, s);
     const int j1 = i == 2 ? 0 : i + 1, j2 = i == 0 ? 2 : i - 1;
     const Q Uj1 = W.load(j1, s), Uj2 = W.load(j2, s);
@@ -333,7 +336,7 @@ __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double 
         qacc<true, false>(S, qmul<false, false>(load(i, s + bj), load(j, pi + bj)), load(j, s + bj));
     }
     if (worst == LINK_BAD) return false;
-    finish_link<HAS_J, I>(small, Ui, S, U, E, J, Unext, L, s, i);
+    finish_link<HAS_J, I>(small, Ui, S, U, E, J, Unext, Unf, L, s, i);
     return true;
 }
 
@@ -341,7 +344,7 @@ __device__ __forceinline__ bool update_link(const FxLinks<2, I> W, const double 
 // staple plane rolled
 template <bool HAS_J, typename I>
 __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double *__restrict__ U, double *__restrict__ E,
-                                            const double *__restrict__ J, double *__restrict__ Unext, const Lat &L, I s, int i) {
+                                            const double *__restrict__ J, double *Unext, int2 *__restrict__ Unf, const Lat &L, I s, int i) {
     int x[3];
     site_coords<I>(L, s, x);
     const Deltas<I> D = deltas<I>(L, x);
@@ -440,8 +443,15 @@ __device__ __forceinline__ bool update_link(const FxLinks<3, I> W, const double 
             }
         }
         Un.store(i, s, V);
+        if (Unf) {
+            double u[18];
+#pragma unroll
+            for (int c = 0; c < 9; c++) { u[c] = V.r[c]; u[9 + c] = V.i[c]; }
+            write_fixed<3, I>(u, Unf, (I)L.V, i, s);
+        }
     } else {
         link_update_f64<3, I>(U, Unext, L, s, i, e);
+        if (Unf) fixed_link<3, double, I>(Unext, Unf, (I)L.V, i, s);
     }
     return true;
 }
@@ -461,10 +471,11 @@ k_update_links_fx(const int2 *__restrict__ Uf, const double *__restrict__ U, dou
     const I s = (I)chunk * (I)blockDim.x + (I)threadIdx.x;
     if (s >= (I)L.V) return;
     if (active && !active[s]) return;  // Cell.isActive gate (FastTYMSolver.java:51)
-    if (!update_link<HAS_J, I>(FxLinks<NC, I>{Uf, (I)L.V}, U, E, J, Unext, L, s, i))
+    // the new link in fixed point too, from the doubles that are stored
+    if (!update_link<HAS_J, I>(FxLinks<NC, I>{Uf, (I)L.V}, U, E, J, Unext, Unf, L, s, i)) {
         update_link_f64<HAS_J, I>(LinkPlanes<typename GroupOf<NC, double>::T, double, I>{const_cast<double *>(U), (I)L.V}, E, J, Unext, L, s, i);
-    // the new link in fixed point, from the double that was stored
-    if (Unf) fixed_link<NC, double, I>(Unext, Unf, (I)L.V, i, s);
+        if (Unf) fixed_link<NC, double, I>(Unext, Unf, (I)L.V, i, s);
+    }
 }
 
 }  // namespace fx
