@@ -204,7 +204,7 @@ int opx_create(const opx_config *cfg, opx_ctx **out) {
     if (ok && (cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess)) ok = false;
     // without room for the fixed-point links the handle works all the same, in FP64 products,
     // and what it allocates later may have theirs (dev_malloc).  Other handles' allocations
-    // find that much less: 192 B a site for SU(2), 876 for SU(3)
+    // find that much less: 192 B a site for SU(2), 888 for SU(3)
     const size_t fxb = fx::fixed_links_bytes(V, c.ng);
     if (ok && c.fixed_kernel && (cudaMalloc(&c.fx_U, fxb) != cudaSuccess || cudaMalloc(&c.fx_Unext, fxb) != cudaSuccess)) {
         cudaGetLastError();

@@ -357,7 +357,7 @@ static cudaError_t launch_flat(Batch &b, int nsteps, cudaStream_t st) {
         void *args[] = {(void *)&ev, (void *)&order, (void *)&bstart, (void *)&nev, (void *)&rd, (void *)&cold};
         void *kf = b.int_offsets ? (reunit ? flat_kernel<NC, R, int, true>() : flat_kernel<NC, R, int, false>())
                                  : (reunit ? flat_kernel<NC, R, long, true>() : flat_kernel<NC, R, long, false>());
-        // the steps overlap as in launch_pdl (in a captured graph too)
+        // the steps overlap as in launch_pdl, from 456 blocks on (in a captured graph too)
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(b.flat_blocks);
         cfg.blockDim = dim3(b.block);

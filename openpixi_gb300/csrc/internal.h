@@ -20,8 +20,9 @@ namespace opx {
 // 2 to 3 us a step (SU(2) FP32 64^3 0.0123 -> 0.0098 ms, 128^3 0.0804 -> 0.0779).
 // A grid of about one block per SM must not: its blocks would go, several to an SM,
 // to the few SMs that its predecessor leaves free (SU(3) FP64 16^3, 96 blocks:
-// 0.025 -> 0.048 ms; 18^3 to 26^3 likewise), so only grids of three blocks per SM or
-// more and those of at most a third of the SMs overlap, or, light, those of short kernels.
+// 0.025 -> 0.048 ms; 18^3 to 26^3 likewise).  So grids of 49 to 455 blocks do not
+// overlap, whatever the kernel's occupancy (the two counts are from blocks of 96 to 192
+// threads, three to eight of them resident on an SM), but for, light, those of short kernels.
 template <typename... P, typename... A>
 inline void launch_pdl(bool light, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {
     cudaLaunchConfig_t cfg = {};
@@ -100,8 +101,9 @@ struct Ctx {
     bool stream_kernel = false;
     int st_grid = 0;
     // FP64: the group products of the update and the reductions in fixed point
-    // (fixed.cuh) where the lattice spacings are equal; OPX_FP64_ONLY=1 keeps every
-    // product in FP64, so that tests can compare the two.  fx_U, fx_Unext: U and
+    // (fixed.cuh) where the lattice spacings are equal; OPX_FP64_ONLY=1 at creation keeps
+    // every product in FP64, so that tests can compare the two (batches and
+    // opx_reduce_noalloc follow it too).  fx_U, fx_Unext: U and
     // Unext in fixed point beside the doubles (swapped with them); fx_*_ok: whether
     // they hold the present links (cleared by every entry point that may write
     // links otherwise than the fixed-point update does)

@@ -22,16 +22,16 @@
 // the FP64 products by chance makes the whole grid wait (SU(3) 40^3 0.130 ms, with
 // 2^-10 0.181): at a width of 0.05 it is one link in 10^7 (SU(2): 10^8).
 //
-// Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.291 ms
-// a step, 128^3 2.014 -> 0.575, SU(3) 64^3 2.99 -> 0.492 ms (the FP64 pipe before);
-// 32^3 0.041 -> 0.018 ms (0.014 with overlapped launches) and SU(3) 16^3 0.221 ->
-// 0.027 ms, where a thread's serial chain counts: one link per thread is a third of
+// Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.288 ms
+// a step, 128^3 2.014 -> 0.568, SU(3) 64^3 2.99 -> 0.477 ms (the FP64 pipe before);
+// 32^3 0.041 -> 0.018 ms (0.0134 with overlapped launches) and SU(3) 16^3 0.221 ->
+// 0.0246 ms, where a thread's serial chain counts: one link per thread is a third of
 // it, and beats one site per thread with the forward staples of a plane sharing a
 // product (21 instead of 24 products for a site) at every size tried (SU(2) 16^3
 // 0.0123 against 0.0184 ms, 128^3 0.728 against 0.773, both before the asm
 // multiply-adds).
 // SU(3) by whole matrix products at 168 registers: 64^3 0.727 against 0.681 ms row
-// by row at 128 (both before the multiply-adds were written in asm, 0.492).
+// by row at 128 (both before the multiply-adds were written in asm).
 #pragma once
 #include "fixed.cuh"
 #include "internal.h"

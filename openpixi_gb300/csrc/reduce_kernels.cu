@@ -14,7 +14,9 @@
 //       fixed point (fixed.cuh), three warps for 32 sites
 //   k_energy_density   : EnergyDensity.ComponentComputation (EnergyDensity.java:119-166)
 //   k_projected_energy : ProjectedEnergyDensity.EnergyDensityComputation (:114-179)
-//   k_gauss_field      : Grid.getGaussConstraint (Grid.java:944-968) at every cell
+//   k_gauss_field      : Grid.getGaussConstraint (Grid.java:944-968) at every cell, in the
+//       storage precision's own products (FP64: the sum of its squares differs from the
+//       BulkQuantities column, whose transports are in fixed point, by rounding)
 #include <algorithm>
 
 #include "internal.h"
