@@ -343,7 +343,11 @@ static int implicit_update_t(Ctx &c) {
     if (!c.imp_Ua) {
         if (dev_malloc(c, &c.imp_Ua, nU) != cudaSuccess || dev_malloc(c, &c.imp_Ub, nU) != cudaSuccess ||
             dev_malloc(c, &c.imp_E, nE) != cudaSuccess) {
-            cudaGetLastError();
+            // all three or none: the next step tries again
+            for (void **p : {&c.imp_Ua, &c.imp_Ub, &c.imp_E}) {
+                cudaFree(*p);
+                *p = nullptr;
+            }
             c.err = "implicit solver: out of device memory";
             return OPX_ERR_NOMEM;
         }

@@ -157,3 +157,29 @@ def test_charge_direction_without_room_for_fixed_links(native, prec):
         fill.release()
     # conjugate gradients to 1e-13 of the right side, either way
     assert abs(J - J0) <= 1e-9 * abs(J0)
+
+
+def test_implicit_solver_tries_its_buffers_again(native):
+    """Without room for all of its buffers a step is refused, every time, and works once
+    there is room."""
+    torch = pytest.importorskip("torch")
+    dims = (64, 64, 64)
+    h, ref = (handle(3, dims, prec=N.OPX_F32) for _ in range(2))
+    for x in (h, ref):
+        x.initialize()
+        x.step(1)
+        x.set_field_solver(N.SOLVER_IMPLICIT, 2, 0.5)
+    ref.step(1)
+    links = 64 ** 3 * 3 * 18 * 4  # room for one of the two copies of the links
+    fill = Filler(torch, links + links // 4)
+    try:
+        for _ in range(2):
+            with pytest.raises(opx.OpixiError) as e:
+                h.update_grid()
+            assert e.value.code == N.OPX_ERR_NOMEM
+    finally:
+        fill.release()
+    h.store_fields()
+    h.update_grid()
+    for f in (N.FIELD_UNEXT, N.FIELD_E):
+        assert np.array_equal(h.download(f), ref.download(f))
