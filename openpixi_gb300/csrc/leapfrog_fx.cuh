@@ -22,7 +22,7 @@
 // the FP64 products by chance makes the whole grid wait (SU(3) 40^3 0.130 ms, with
 // 2^-10 0.181): at a width of 0.05 it is one link in 10^7 (SU(2): 10^8).
 //
-// Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.288 ms
+// Bound: the issue slots of the integer pipes.  256 x 64^2 SU(2) 1.014 -> 0.286 ms
 // a step, 128^3 2.014 -> 0.568, SU(3) 64^3 2.99 -> 0.477 ms (the FP64 pipe before);
 // 32^3 0.041 -> 0.018 ms (0.0134 with overlapped launches) and SU(3) 16^3 0.221 ->
 // 0.0246 ms, where a thread's serial chain counts: one link per thread is a third of
